@@ -119,11 +119,16 @@ struct DevNet {
     void *density_state = nullptr;
     void (*density_free)(void *) = nullptr;
 
+    // cached forms of the groups as excitations (rotation sequences)
+    void *rot_state = nullptr;
+    void (*rot_free)(void *) = nullptr;
+
     int finalize();   // derived tables + upload
     ~DevNet() {
         if (fast_state && fast_free) fast_free(fast_state);
         if (pair_state && pair_free) pair_free(pair_state);
         if (density_state && density_free) density_free(density_state);
+        if (rot_state && rot_free) rot_free(rot_state);
         arena.release();
         magic = 0;
     }

@@ -11,12 +11,16 @@
 //     and the reverse sweep restores l from the copy when it reaches that
 //     position, which stops uncompute drift (the Givens rotations are unitary
 //     only to the precision of the SVD weights);
+//   * consecutive components that move the same few orbitals (those of one
+//     spin-adapted generator) are applied in one pass over the state
+//     (rotseq.cu), the others one by one through the pair kernels;
 //   * spin-adapted generators are ordered products of spin-orbital components
 //     sharing one parameter: param_idx maps each applied component to its
 //     parameter and the gradient sums the component terms.
 #include "vqe.h"
 #include "dav.h"
 #include "ops.h"
+#include "rotseq.h"
 
 #include <algorithm>
 #include <cmath>
@@ -65,7 +69,10 @@ int prepare_state(const DevBasis<Ti> *B, const DevNet<Ti> *P, i64 n_ops, const i
         BSIM_CUDA(cudaGetLastError());
         BSIM_CUDA(cudaStreamSynchronize(s));   // host arrays of the copies must outlive them
     }
-    for (i64 i = 0; i < n_ops; ++i) TRY(expm(B, P, op_idx[i], thetas[param_idx[i]], v, s));
+    if (n_ops == 0) return BSIM_OK;
+    RotSequence<Ti> seq;
+    TRY(seq.init(B, P, n_ops, op_idx, param_idx, thetas, {}, s));
+    for (i64 u = 0; u < seq.size(); ++u) TRY(seq.forward(u, v));
     return BSIM_OK;
 }
 
@@ -98,27 +105,36 @@ int vqe_energy_grad(const DevBasis<Ti> *B, const DevNet<Ti> *H, const DevNet<Ti>
 
     // forward: psi_0 = reference, psi_{i+1} = exp(theta G_i) psi_i
     TRY(prepare_state(B, P, 0, op_idx, param_idx, thetas, ref_idx, ref_val, n_ref, lv, s));
+    RotSequence<Ti> seq;
+    TRY(seq.init(B, P, n_ops, op_idx, param_idx, thetas, ck_pos, s));
     size_t c = 0;
-    for (i64 i = 0; i < n_ops; ++i) {
-        if (c < ck_pos.size() && ck_pos[c] == i) {
-            BSIM_CUDA(cudaMemcpyAsync(ckp + (size_t)c * n, lv, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-            ++c;
-        }
-        TRY(expm(B, P, op_idx[i], thetas[param_idx[i]], lv, s));
+    for (i64 u = 0; u < seq.size(); ++u) {
+        for (; c < ck_pos.size() && ck_pos[c] <= seq.unit(u).op0; ++c, seq.unchain())
+            BSIM_CUDA(cudaMemcpyAsync(ckp + c * (size_t)n, lv, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+        TRY(seq.forward(u, lv));
     }
+    const size_t n_saved = c;
+    seq.unchain();
     // energy: r = H l, E = <l|r>/<l|l>
     TRY(sigma(B, H, lv, nullptr, rv, false, s));
     TRY(dav_dot(S, n, lv, lv, sc + 0, s));
     TRY(dav_dot(S, n, lv, rv, sc + 1, s));
     TRY(dav_dot(S, n, rv, rv, sc + 2, s));
     // reverse sweep
-    for (i64 i = n_ops - 1; i >= 0; --i) {
-        TRY(backgrad(B, P, op_idx[i], thetas[param_idx[i]], lv, rv, tp + i, false, s));
-        if (c > 0 && ck_pos[c - 1] == i) {
-            --c;
-            BSIM_CUDA(cudaMemcpyAsync(lv, ckp + (size_t)c * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    BSIM_CUDA(cudaMemsetAsync(tp, 0, sizeof(double) * n_terms, s));   // diagonal groups have no unit
+    c = n_saved;
+    for (i64 u = seq.size() - 1; u >= 0; --u) {
+        TRY(seq.backward(u, lv, rv, tp));
+        // the checkpoint taken before this unit (the first of equal ones)
+        const i64 before = u > 0 ? seq.unit(u - 1).op0 : -1;
+        bool restore = false;
+        for (; c > 0 && ck_pos[c - 1] > before; --c) restore = true;
+        if (restore) {
+            BSIM_CUDA(cudaMemcpyAsync(lv, ckp + c * (size_t)n, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+            seq.unchain();
         }
     }
+    TRY(seq.flush(tp));
     std::vector<double> h_terms(std::max<i64>(1, n_ops)), h_sc(3);
     BSIM_CUDA(cudaMemcpyAsync(h_terms.data(), tp, sizeof(double) * n_ops, cudaMemcpyDeviceToHost, s));
     BSIM_CUDA(cudaMemcpyAsync(h_sc.data(), sc, sizeof(double) * 3, cudaMemcpyDeviceToHost, s));

@@ -119,6 +119,9 @@ struct DevNet {
     void *density_state = nullptr;
     void (*density_free)(void *) = nullptr;
 
+    // cached sigma plan of a symmetry-blocked basis
+    void *blk_state = nullptr;
+    void (*blk_free)(void *) = nullptr;
     // cached forms of the groups as excitations (rotation sequences)
     void *rot_state = nullptr;
     void (*rot_free)(void *) = nullptr;
@@ -129,6 +132,7 @@ struct DevNet {
         if (pair_state && pair_free) pair_free(pair_state);
         if (density_state && density_free) density_free(density_state);
         if (rot_state && rot_free) rot_free(rot_state);
+        if (blk_state && blk_free) blk_free(blk_state);
         arena.release();
         magic = 0;
     }

@@ -25,6 +25,11 @@ i64 num_tiles(const DevBasis<Ti> *B);
 template <typename Ti>
 int sigma_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, const float *src32, double *dst,
                bool mixed, cudaStream_t s, bool *used);
+// Sigma on symmetry-blocked bases through per-row lists (sigma_blocks.cu); *used
+// tells whether it ran.
+template <typename Ti>
+int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, const float *src32, double *dst,
+                 bool mixed, cudaStream_t s, bool *used);
 // 1: structured path (FP64 and FP32), 2: structured for FP32 only, 0: generic.
 // Columns [col_lo, col_hi) of sigma through the structured path (col_lo a
 // multiple of 128): the unit of work of one rank when sigma is split by beta

@@ -211,8 +211,8 @@ int sigma_generic_accumulate(const DevBasis<Ti> *B, const DevNet<Ti> *N, const i
     return BSIM_OK;
 }
 
-// Structured path when the plan accepts the (basis, network) pair, else the
-// generic tile kernel.  BSIM_SIGMA_GENERIC=1 forces the generic kernel.
+// Structured path when the plan accepts the (basis, network) pair, the row lists
+// for a symmetry-blocked basis, else the generic tile kernel.  BSIM_SIGMA_GENERIC=1 forces the generic kernel.
 template <typename Ti>
 int sigma(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, const float *src32, double *dst,
           bool mixed, cudaStream_t s)
@@ -224,6 +224,8 @@ int sigma(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, const f
     if (!force_generic && B->dim > 0) {
         bool used = false;
         int st = sigma_fast(B, N, src, src32, dst, mixed, s, &used);
+        if (st != BSIM_OK) return st;
+        if (!used) st = sigma_blocks(B, N, src, src32, dst, mixed, s, &used);
         if (st != BSIM_OK) return st;
         if (used) return BSIM_OK;
     }

@@ -1,0 +1,63 @@
+"""Sigma on symmetry-blocked bases (per-row lists) against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _masked(norb, sym, seed):
+    """A Hamiltonian whose integrals respect the point group."""
+    from binsim_b200 import network as nw
+    h, g, _ = nw.synthetic_integrals(norb, seed)
+    s = np.asarray(sym)
+    h = h * ((s[:, None] ^ s[None, :]) == 0)
+    g = g * ((s[:, None, None, None] ^ s[None, :, None, None] ^ s[None, None, :, None] ^ s[None, None, None, :]) == 0)
+    x, z, c = nw.jw_hamiltonian_terms(h, g)
+    return nw.compress_groups(*nw.split_aabb(x, z, norb), c, norb, orbsym=s)
+
+
+# electron counts at the ends, unequal spins, odd irreps, one- and two-block bases, rows longer than a CTA's 128 columns
+@pytest.mark.parametrize("norb,na,nb,sym,nirr,tsym,bits", [
+    (4, 1, 3, [0, 1, 0, 1], 2, 1, 32), (5, 0, 2, [0, 1, 1, 0, 1], 2, 0, 32), (6, 6, 1, [0, 1, 2, 3, 0, 1], 4, 2, 64),
+    (9, 4, 5, [0, 1, 2, 3, 4, 5, 6, 7, 0], 8, 5, 32), (11, 5, 6, [0, 0, 1, 1, 0, 1, 0, 0, 1, 1, 0], 2, 1, 32),
+    (10, 5, 5, [0, 1, 2, 3, 0, 1, 2, 3, 0, 1], 4, 0, 64)])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_blocked_sigma(cuda, oracle, norb, na, nb, sym, nirr, tsym, bits, symmetric):
+    from binsim_b200 import cuotf, network as nw
+    sym = np.asarray(sym, np.int64)
+    if symmetric:
+        net = _masked(norb, sym, norb)
+    else:   # integrals of every irrep: the terms that leave the total irrep drop out
+        net = nw.hamiltonian_network(norb, seed=norb)
+        net.orbsym = sym
+    kw = dict(orbsym=sym, total_sym=tsym, num_irreps=nirr)
+    Bo, No = oracle.basis(norb, na, nb, **kw), oracle.network(net)
+    B = cuotf.CuBasis(norb, na, nb, string_bits=bits, **kw)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net, string_bits=bits))
+    assert B.dim == Bo.dim and f.sigma_path()[0] == 0
+    x = np.random.default_rng(norb).normal(size=B.dim)
+    ref = oracle.hvec(Bo, No, x)
+    scale = max(np.abs(ref).max(), 1e-300)
+    for call, tol in ((f.hvec, 1e-13), (f.hvec_mixed, 2e-6)):
+        y = cuda.full((B.dim,), float("nan"), dtype=cuda.float64, device="cuda")
+        call(dev(cuda, x), y)
+        assert np.abs(y.cpu().numpy() - ref).max() <= tol * scale
+
+
+def test_blocked_sigma_with_other_groups(cuda, oracle):
+    """Groups that are no part of a two-body Hamiltonian (antisymmetric generators) go through the tile kernel."""
+    from binsim_b200 import cuotf, network as nw
+    norb, na, nb, sym = 6, 3, 2, np.array([0, 1, 0, 1, 1, 0], np.int64)
+    net = nw.ucc_pool(norb).network
+    net.orbsym = sym
+    kw = dict(orbsym=sym, total_sym=1, num_irreps=2)
+    Bo, No = oracle.basis(norb, na, nb, **kw), oracle.network(net)
+    B = cuotf.CuBasis(norb, na, nb, **kw)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+    x = np.random.default_rng(1).normal(size=B.dim)
+    ref = oracle.hvec(Bo, No, x)
+    y = cuda.empty(B.dim, dtype=cuda.float64, device="cuda")
+    f.hvec(dev(cuda, x), y)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()

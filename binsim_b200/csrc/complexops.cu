@@ -10,14 +10,19 @@
 //
 // Kernels: one CTA per destination alpha row of every block, lanes over the
 // row's beta columns (the row-pair scheme of the real operators in
-// pairops.cu, with the reference's once-per-pair rule); sigma loops over all
-// groups inside the CTA, so each CTA owns its destination row and needs no
-// atomics.  Scalar results reduce deterministically through per-CTA partials
-// summed in slot order by the last CTA.
+// pairops.cu, with the reference's once-per-pair rule); sigma walks per-row lists of
+// the connected groups with tabled partners and phases, or, where those would be
+// too large, loops over all groups inside a row's CTA; no atomics in either.
+// Scalar results reduce deterministically through per-CTA partials summed in slot
+// order by the last CTA.
 #include "../../include/binsim_cuotf.h"
 #include "ops.h"
 
+#include <algorithm>
 #include <cmath>
+#include <mutex>
+#include <unordered_map>
+#include <vector>
 
 namespace bsim {
 
@@ -104,6 +109,258 @@ c64_hvec_kernel(const BasisView<Ti> B, const NetView<Ti> N, const cx *__restrict
         }
         if (b < nb) dst[drow + b] = acc;
     }
+}
+
+// ---- sigma over lists: the same sum with partners and phases tabled once ------------
+// One entry per (alpha row, connected group, rank index r): the source row, the
+// group's beta partner table and beta phase row, and PA_r of the source string.  A
+// CTA of 8 warps owns 32 columns of a row; each warp adds every eighth entry, the
+// warps' sums are added in order.  Bound: L1 (per entry and column 4 + 16 + 16
+// bytes).  c64_hvec_kernel, one CTA per row with every partner and phase found on
+// the way, left most of the chip idle: 3.43 ms at 10o 5a+5b against 0.31 ms.
+struct C64Ent {
+    long long srow;      // source row offset
+    int part, ph;        // first entry of the partner table / of the phase row
+    cx pa;
+};
+constexpr int kC64Cols = 32;
+constexpr size_t kC64Tables = (size_t)1 << 30;   // larger lists: the row kernel
+
+// partner tables: row m of mask masks[m] over every beta string (local index or -1)
+template <typename Ti>
+__global__ void c64_partner_kernel(const BasisView<Ti> B, int nBt, const u64 *__restrict__ masks, int *__restrict__ part)
+{
+    const u64 x = masks[blockIdx.y];
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nBt; b += gridDim.x * blockDim.x)
+        part[(i64)blockIdx.y * nBt + b] = string_index(B, B.bmap, B.nel_b, (Ti)((u64)B.bstrs[b] ^ x));
+}
+
+// phase rows: row prow[g] + r holds PB_r of group g at the source string of every beta string
+template <typename Ti>
+__global__ void c64_phase_kernel(const BasisView<Ti> B, const NetView<Ti> N, int nBt, const int *__restrict__ prow,
+                                 cx *__restrict__ ph)
+{
+    const GroupDev g = N.g[blockIdx.y];
+    const cx *W = reinterpret_cast<const cx *>(N.w);
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nBt; b += gridDim.x * blockDim.x)
+        for (int r = 0; r < g.rank; ++r)
+            ph[(i64)(prow[blockIdx.y] + r) * nBt + b] =
+                cphase((u64)B.bstrs[b] ^ g.bx, N.z + g.zb_off, g.nzb, W + g.wb_off + (i64)r * g.nzb);
+}
+
+// entries of one row per CTA; ent == nullptr: count them only
+template <typename Ti>
+__global__ void __launch_bounds__(kC64Threads)
+c64_entries_kernel(const BasisView<Ti> B, const NetView<Ti> N, int nBt, const int2 *__restrict__ row,
+                   const int *__restrict__ mask_of, const int *__restrict__ prow, const i64 *__restrict__ start,
+                   int *__restrict__ count, C64Ent *__restrict__ ent)
+{
+    __shared__ int wsum[kC64Threads / 32];
+    const int kd = row[blockIdx.x].x, a = row[blockIdx.x].y;
+    const cx *W = reinterpret_cast<const cx *>(N.w);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    i64 at = ent ? start[blockIdx.x] : 0;
+    for (int base = 0; base < N.ngs; base += kC64Threads) {
+        const int gi = base + threadIdx.x;
+        int ks = -1, sa = -1, n = 0;
+        Ti s_a = 0;
+        if (gi < N.ngs && source_row(B, N.g[gi], kd, a, false, &ks, &sa, &s_a)) n = N.g[gi].rank;
+        int inc = n;   // inclusive prefix of the entries in group order
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane == 31) wsum[wid] = inc;
+        __syncthreads();
+        int before = 0, total = 0;
+        for (int w = 0; w < kC64Threads / 32; ++w) {
+            if (w < wid) before += wsum[w];
+            total += wsum[w];
+        }
+        __syncthreads();
+        if (ent && n > 0) {
+            const GroupDev g = N.g[gi];
+            for (int r = 0; r < n; ++r)
+                ent[at + before + inc - n + r] =
+                    C64Ent{B.blk_off[ks] + (i64)sa * B.blk_nb[ks], mask_of[gi] * nBt, prow[gi] + r,
+                           cphase(s_a, N.z + g.za_off, g.nza, W + g.wa_off + (i64)r * g.nza)};
+        }
+        at += total;
+    }
+    if (!ent && threadIdx.x == 0) count[blockIdx.x] = (int)at;
+}
+
+template <typename Ti>
+__global__ void __launch_bounds__(kC64Threads)
+c64_list_hvec_kernel(const BasisView<Ti> B, int nBt, const int2 *__restrict__ row, const i64 *__restrict__ start,
+                     const C64Ent *__restrict__ ent, const int *__restrict__ part, const cx *__restrict__ ph,
+                     const cx *__restrict__ src, cx *__restrict__ dst)
+{
+    constexpr int NW = kC64Threads / 32;
+    __shared__ double2 red[NW][kC64Cols];
+    const int kd = row[blockIdx.x].x, a = row[blockIdx.x].y, nb = B.blk_nb[kd];
+    if ((int)blockIdx.y * kC64Cols >= nb) return;   // uniform across the CTA
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int b = blockIdx.y * kC64Cols + lane;
+    const int gb = B.blk_bstart[kd] + min(b, nb - 1);
+    const double2 *ph2 = reinterpret_cast<const double2 *>(ph), *src2 = reinterpret_cast<const double2 *>(src);
+    cx acc = {0.0, 0.0};
+    const i64 e1 = start[blockIdx.x + 1];
+#pragma unroll 4
+    for (i64 e = start[blockIdx.x] + wid; e < e1; e += NW) {
+        const C64Ent x = ent[e];
+        const int sb = __ldg(part + x.part + gb);
+        if (sb < 0) continue;
+        const double2 p = __ldg(ph2 + (i64)x.ph * nBt + gb), v = __ldg(src2 + x.srow + sb);
+        acc = cadd(acc, cmul(cx{v.x, v.y}, cmul(x.pa, cx{p.x, p.y})));   // hvec_update, core/math.hpp:126-130
+    }
+    red[wid][lane] = make_double2(acc.x, acc.y);
+    __syncthreads();
+    if (wid == 0 && b < nb) {
+        for (int w = 1; w < NW; ++w) acc = cadd(acc, cx{red[w][lane].x, red[w][lane].y});
+        dst[B.blk_off[kd] + (i64)a * nb + b] = acc;
+    }
+}
+
+// lists of one (basis, network), built with the first sigma
+struct C64Lists {
+    const void *basis = nullptr;
+    i64 dim = -1;
+    bool ok = false;
+    int nBt = 0, nrows = 0, ytiles = 0;
+    Arena arena;
+    const int2 *row = nullptr;
+    const i64 *start = nullptr;
+    const C64Ent *ent = nullptr;
+    const int *part = nullptr;
+    const cx *ph = nullptr;
+    ~C64Lists() { arena.release(); }
+};
+
+std::mutex g_c64_mu;
+
+template <typename Ti>
+int c64_build(const DevBasis<Ti> *B, const DevNet<Ti> *N, C64Lists *P, cudaStream_t s)
+{
+    P->basis = B;
+    P->dim = B->dim;
+    P->ok = false;
+    if (N->ngs == 0 || N->ngs > 65535 || B->dim == 0) return BSIM_OK;
+    std::vector<int2> row;
+    for (int k = 0; k < B->num_blocks; ++k)
+        for (int a = 0; a < B->na[k]; ++a) row.push_back(make_int2(k, a));
+    P->nBt = (int)B->bstrs.size();
+    P->nrows = (int)row.size();
+    P->ytiles = (B->max_nb + kC64Cols - 1) / kC64Cols;
+    std::unordered_map<u64, int> mid;
+    std::vector<u64> masks;
+    std::vector<int> mask_of, prow;
+    i64 rows = 0;
+    for (const GroupDev &G : N->groups) {
+        auto it = mid.find(G.bx);
+        if (it == mid.end()) {
+            it = mid.emplace(G.bx, (int)masks.size()).first;
+            masks.push_back(G.bx);
+        }
+        mask_of.push_back(it->second);
+        prow.push_back((int)rows);
+        rows += G.rank;
+    }
+    const double tables = (double)P->nBt * ((double)rows * sizeof(cx) + (double)masks.size() * 4);
+    if (tables > (double)kC64Tables || (double)masks.size() * P->nBt > 2e9 || masks.size() > 65535 || P->ytiles > 65535)
+        return BSIM_OK;
+    // count the entries of every row
+    auto al = [](size_t n) { return (n + 255) & ~size_t(255); };
+    const size_t small = al(row.size() * 8) + al(masks.size() * 8) + 2 * al(mask_of.size() * 4) + al(row.size() * 4);
+    char *tmp = nullptr;
+    cudaError_t e = dmalloc(&tmp, small);
+    if (e == cudaErrorMemoryAllocation) { (void)cudaGetLastError(); return BSIM_ERR_ALLOC; }   // the row kernel serves
+    if (e != cudaSuccess) return cuda_status(e, "complex sigma lists");
+    char *p = tmp;
+    auto up = [&](const auto &v) {
+        auto *d = reinterpret_cast<const typename std::decay_t<decltype(v)>::value_type *>(p);
+        if (e == cudaSuccess) e = cudaMemcpy(p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice);
+        p += al(v.size() * sizeof(v[0]));
+        return d;
+    };
+    const int2 *d_row = up(row);
+    const u64 *d_masks = up(masks);
+    const int *d_mask_of = up(mask_of), *d_prow = up(prow);
+    int *d_count = reinterpret_cast<int *>(p);
+    std::vector<int> count(row.size());
+    std::vector<i64> start(row.size() + 1, 0);
+    if (e == cudaSuccess) {
+        c64_entries_kernel<Ti><<<P->nrows, kC64Threads, 0, s>>>(B->view, N->view, P->nBt, d_row, d_mask_of, d_prow, nullptr,
+                                                               d_count, nullptr);
+        e = cudaMemcpyAsync(count.data(), d_count, count.size() * 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    }
+    for (size_t i = 0; i < row.size(); ++i) start[i + 1] = start[i] + count[i];
+    int st = BSIM_OK;
+    const bool fits = tables + (double)start.back() * sizeof(C64Ent) <= (double)kC64Tables;
+    if (e == cudaSuccess && fits) {
+        st = P->arena.reserve(al(row.size() * 8) + al(start.size() * 8) + al((size_t)start.back() * sizeof(C64Ent) + 1) +
+                              al(masks.size() * P->nBt * 4) + al((size_t)rows * P->nBt * sizeof(cx) + 1));
+        if (st == BSIM_OK) {
+            int2 *r2 = P->arena.take<int2>(row.size());
+            i64 *s2 = P->arena.take<i64>(start.size());
+            C64Ent *en = P->arena.take<C64Ent>((size_t)start.back());
+            int *pt = P->arena.take<int>(masks.size() * P->nBt);
+            cx *ph = P->arena.take<cx>((size_t)rows * P->nBt);
+            e = cudaMemcpy(r2, row.data(), row.size() * 8, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = cudaMemcpy(s2, start.data(), start.size() * 8, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) {
+                const unsigned bx = (unsigned)std::min(64, (P->nBt + 255) / 256);
+                c64_partner_kernel<Ti><<<dim3(bx, (unsigned)masks.size()), 256, 0, s>>>(B->view, P->nBt, d_masks, pt);
+                c64_phase_kernel<Ti><<<dim3(bx, (unsigned)N->ngs), 256, 0, s>>>(B->view, N->view, P->nBt, d_prow, ph);
+                c64_entries_kernel<Ti><<<P->nrows, kC64Threads, 0, s>>>(B->view, N->view, P->nBt, r2, d_mask_of, d_prow,
+                                                                       s2, nullptr, en);
+                e = cudaGetLastError();
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // the group tables are freed below
+            }
+            P->row = r2; P->start = s2; P->ent = en; P->part = pt; P->ph = ph;
+            P->ok = true;
+        }
+    }
+    cudaFree(tmp);
+    if (st == BSIM_ERR_ALLOC) (void)cudaGetLastError();
+    if (e != cudaSuccess) return cuda_status(e, "complex sigma lists");
+    return st;
+}
+
+template <typename Ti>
+int c64_hvec(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, double *dst, cudaStream_t s)
+{
+    if (B->dim == 0) return BSIM_OK;
+    C64Lists *P = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_c64_mu);
+        P = static_cast<C64Lists *>(N->c64_state);
+        if (P && (P->basis != B || P->dim != B->dim)) {
+            delete P;
+            P = nullptr;
+            const_cast<DevNet<Ti> *>(N)->c64_state = nullptr;
+        }
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (!P) BSIM_CUDA(cudaStreamIsCapturing(s, &cap));
+        if (!P && cap == cudaStreamCaptureStatusNone) {   // building allocates and waits: not inside a capture
+            P = new C64Lists();
+            const int st = c64_build(B, N, P, s);
+            if (st != BSIM_OK && st != BSIM_ERR_ALLOC) { delete P; return st; }
+            const_cast<DevNet<Ti> *>(N)->c64_state = P;
+            const_cast<DevNet<Ti> *>(N)->c64_free = [](void *q) { delete static_cast<C64Lists *>(q); };
+        }
+    }
+    const cx *x = reinterpret_cast<const cx *>(src);
+    cx *y = reinterpret_cast<cx *>(dst);
+    if (P && P->ok)
+        c64_list_hvec_kernel<Ti><<<dim3((unsigned)P->nrows, (unsigned)P->ytiles), kC64Threads, 0, s>>>(
+            B->view, P->nBt, P->row, P->start, P->ent, P->part, P->ph, x, y);
+    else
+        c64_hvec_kernel<Ti><<<dim3(B->max_na, B->num_blocks), kC64Threads, 0, s>>>(B->view, N->view, x, y);
+    BSIM_CUDA(cudaGetLastError());
+    return BSIM_OK;
 }
 
 // ---- one group: the pair operators ---------------------------------------------
@@ -368,12 +625,7 @@ int bsim_hvec_c64(void *basis, void *net, const double *src, double *dst, bsim_s
 {
     return bsim::with_c64(basis, net, [&](auto *b, auto *n) -> int {
         NEED64(src); NEED64(dst);
-        if (b->dim == 0) return BSIM_OK;
-        dim3 grid(b->max_na, b->num_blocks);
-        bsim::c64_hvec_kernel<<<grid, bsim::kC64Threads, 0, stream>>>(b->view, n->view, reinterpret_cast<const bsim::cx *>(src),
-                                                          reinterpret_cast<bsim::cx *>(dst));
-        BSIM_CUDA(cudaGetLastError());
-        return BSIM_OK;
+        return bsim::c64_hvec(b, n, src, dst, stream);
     });
 }
 

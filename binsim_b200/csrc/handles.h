@@ -119,6 +119,9 @@ struct DevNet {
     void *density_state = nullptr;
     void (*density_free)(void *) = nullptr;
 
+    // cached row lists of the complex sigma
+    void *c64_state = nullptr;
+    void (*c64_free)(void *) = nullptr;
     // cached sigma plan of a symmetry-blocked basis
     void *blk_state = nullptr;
     void (*blk_free)(void *) = nullptr;
@@ -133,6 +136,7 @@ struct DevNet {
         if (density_state && density_free) density_free(density_state);
         if (rot_state && rot_free) rot_free(rot_state);
         if (blk_state && blk_free) blk_free(blk_state);
+        if (c64_state && c64_free) c64_free(c64_state);
         arena.release();
         magic = 0;
     }

@@ -73,6 +73,33 @@ inline cudaError_t dmalloc_async(T **p, size_t bytes, cudaStream_t s)
         if (e__ != cudaSuccess) return ::bsim::cuda_status(e__, #call); \
     } while (0)
 
+// Chained launches (programmatic dependent launch): the kernel's CTAs may become
+// resident while the stream's previous kernel finishes; chain_wait(), before the
+// kernel touches anything an earlier one wrote, waits until that kernel has
+// completed and its writes are visible, and lets the next one start in the same way.
+// Every kernel launched like this calls it first, so the stream's order holds; it
+// hides the launch latency of a sigma's short kernels.
+template <typename... KArgs, typename... Args>
+inline void launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args &&...args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);   // an error stays for cudaGetLastError
+}
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- device views -----------------------------------------------------------
 constexpr int kMaxRank = 64;      // ranks above this are rejected at network build
 constexpr int kMaxIrreps = 16;

@@ -31,6 +31,7 @@
 namespace bsim {
 
 constexpr int kRowChunk = 1024;        // columns per CTA in the row kernels (256 threads x 4)
+constexpr int kSplitCtas = 512;        // below this many CTAs of the row kernel: pure_split_kernel (measured there)
 
 template <typename T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
@@ -56,6 +57,7 @@ __global__ void frame_transpose_kernel(int nA, int nB, int ldA, int ldB, const T
                                        const u64 *__restrict__ Ka, const Tin *__restrict__ c, T *__restrict__ ct,
                                        T *__restrict__ ctT)
 {
+    chain_wait();
     __shared__ T tile[32][33];
     const int b0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -88,6 +90,7 @@ pure_rows_kernel(int row_begin, int col_begin, int ncols, int ld_in, const SideC
                  double *__restrict__ out, int ld_out, const double *__restrict__ PAd, const double *__restrict__ PBdT,
                  int rank_d)
 {
+    chain_wait();
     const int row = row_begin + blockIdx.x;
     const int c = col_begin + blockIdx.y * kRowChunk + 4 * threadIdx.x;
     if (c >= ncols) return;
@@ -177,6 +180,108 @@ pure_rows_kernel(int row_begin, int col_begin, int ncols, int ld_in, const SideC
 #pragma unroll
     for (int k = 0; k < 4; ++k)
         if (c + k < ncols) o[k] = acc[k];
+}
+
+// The same sums with a row's entries divided among the CTA's eight warps (entry e
+// to warp e % 8, the warps' sums added in order), 128 columns per CTA: for sizes
+// that leave pure_rows_kernel a few CTAs per SM, each walking its entries one
+// dependent load after another.  Alpha + beta rows, us, FP64, by the CTAs of the
+// other kernel: 38.4 -> 17.3 at 8o (70), 51.9 -> 27.6 at 10o (252), 62.9 -> 55.6 at
+// 11o 5+5 (462); 154.7 -> 150.3 at 12o 5+5 (792); 172.5 -> 192.9 at 12o 6+6 (924),
+// where the column tables read by every CTA of a row cost more than the waits.
+constexpr int kSplitCols = 128;
+template <typename T>
+__global__ void __launch_bounds__(256)
+pure_split_kernel(int row_begin, int col_begin, int ncols, int ld_in, const SideCSR L, const T *__restrict__ in,
+                  double *__restrict__ out, int ld_out, const double *__restrict__ PAd, const double *__restrict__ PBdT,
+                  int rank_d)
+{
+    chain_wait();
+    constexpr int NW = 8;
+    __shared__ double red[NW][kSplitCols];
+    const int row = row_begin + blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int c0 = col_begin + blockIdx.y * kSplitCols, c = c0 + 4 * lane;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (c < ncols) {
+        const T *in_c = in + c;
+        if (PAd) {
+            T self[4];
+            load4(in_c + (i64)row * ld_in, self);
+            double d[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int r = wid; r < rank_d; r += NW) {
+                const double pa = __ldg(PAd + (i64)row * rank_d + r);
+                double pb[4];
+                load4(PBdT + (i64)r * ld_in + c, pb);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) d[k] += pa * pb[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] = d[k] * (double)self[k];
+        }
+        constexpr int kBatch = 64 * NW;   // FP32 partial sums span at most 64 entries
+        for (i64 e0 = L.cptr[row] + wid; e0 < L.cptr[row + 1]; e0 += kBatch) {
+            const i64 e1 = min(L.cptr[row + 1], e0 + kBatch);
+            T part[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+            for (i64 e = e0; e < e1; e += NW) {
+                const CEnt E = L.cent[e];
+                T v[4];
+                load4(in_c + E.off, v);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) part[k] += (T)E.coef * v[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] += (double)part[k];
+        }
+        const T *ctab = std::is_same<T, float>::value ? reinterpret_cast<const T *>(L.ctab32)
+                                                      : reinterpret_cast<const T *>(L.ctab);
+        const i64 t_end = L.tptr[row + 1];
+#pragma unroll 2
+        for (i64 e = L.tptr[row] + wid; e < t_end; e += NW) {
+            const TEnt t = L.tent[e];
+            const int R = (int)(t.toff_rank & 7);
+            const T *tab = ctab + (t.toff_rank & ~7ll) + c;
+            T v[4], cr[kSideMaxRank][4];
+            load4(in_c + t.off, v);
+#pragma unroll
+            for (int r = 0; r < kSideMaxRank; ++r)
+                if (r < R) load4(tab + (i64)r * ld_in, cr[r]);
+            double f[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int r = 0; r < kSideMaxRank; ++r)
+                if (r < R) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) f[k] += t.pa[r] * (double)cr[r][k];
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] += f[k] * (double)v[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) red[wid][4 * lane + k] = acc[k];
+    __syncthreads();
+    const int t = threadIdx.x;
+    if (t < kSplitCols && c0 + t < ncols) {
+        double v = red[0][t];
+#pragma unroll
+        for (int w = 1; w < NW; ++w) v += red[w][t];
+        out[(i64)row * ld_out + c0 + t] = v;
+    }
+}
+
+template <typename T>
+static void launch_pure(int row0, int row1, int c0, int c1, int ld_in, const SideCSR &L, const T *in, double *out,
+                        int ld_out, const double *PAd, const double *PBdT, int rank_d, cudaStream_t s)
+{
+    const i64 ctas = (i64)(row1 - row0) * ((c1 - c0 + kRowChunk - 1) / kRowChunk);
+    if (row1 <= row0 || c1 <= c0) return;
+    if (ctas < kSplitCtas) {
+        dim3 g(row1 - row0, (c1 - c0 + kSplitCols - 1) / kSplitCols);
+        launch_chained(pure_split_kernel<T>, g, 256, 0, s, row0, c0, c1, ld_in, L, in, out, ld_out, PAd, PBdT, rank_d);
+    } else {
+        dim3 g(row1 - row0, (c1 - c0 + kRowChunk - 1) / kRowChunk);
+        launch_chained(pure_rows_kernel<T>, g, 256, 0, s, row0, c0, c1, ld_in, L, in, out, ld_out, PAd, PBdT, rank_d);
+    }
 }
 
 // ---- 4a. mixed GEMM -----------------------------------------------------------------
@@ -526,6 +631,7 @@ __global__ void __launch_bounds__(512, 1)
 mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *__restrict__ ct,
                   double *__restrict__ Z, int z0, int W, int jbase)
 {
+    chain_wait();
     constexpr int NT = 512;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = P.nF, M = P.M;
@@ -626,6 +732,7 @@ __global__ void __launch_bounds__(256)
 mixed_gather_kernel(const MixedArgs P, const BasisView<Ti> BV, const T *__restrict__ Z, double *__restrict__ sig,
                     int z0, int W)
 {
+    chain_wait();
     __shared__ int esrc[kMaxConn], ej[kMaxConn];
     __shared__ int wcnt[8], cnt;
     const int a = blockIdx.x;
@@ -801,6 +908,7 @@ inline size_t ri_dmma_smem(int nU) { return (size_t)((nU + 31) & ~31) * kRiLS * 
 __global__ void __launch_bounds__(512, 1)
 ri_dmma_kernel(const RIArgs P, const double *__restrict__ in, double *__restrict__ Z, int z0, int W)
 {
+    chain_wait();
     constexpr int NT = 512, MAXRB = (kRiMaxU + 15) / 16;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = P.nU, Kp = (K + 31) & ~31;
@@ -890,6 +998,7 @@ __global__ void __launch_bounds__(256)
 ri_gather_kernel(const RIArgs P, const int2 *__restrict__ gath, const T *__restrict__ Z, double *__restrict__ out,
                  int ld_out, int z0, int W)
 {
+    chain_wait();
     __shared__ long long eoff[64];
     const int row = blockIdx.x;
     for (int e = threadIdx.x; e < P.npr; e += blockDim.x) {
@@ -917,6 +1026,7 @@ template <typename Ti>
 __global__ void final_kernel(int nA, int nB, int ldB, int col_begin, int col_end, const Ti *__restrict__ bstr,
                              const u64 *__restrict__ Ka, const double *__restrict__ tT, double *__restrict__ sig)
 {
+    chain_wait();
     __shared__ double tile[32][33];
     const int b0 = col_begin + blockIdx.x * 32, a0 = blockIdx.y * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -1097,7 +1207,7 @@ static int launch_mixed_shape(const DevBasis<Ti> *B, FastPlan<Ti> &P, const Mixe
         for (int pass = 0; pass < passes; ++pass)
             STAGE(tm, 3, s, (kern<<<P.nA, NT, smem, s>>>(ma, P.d_astr, ct, Z, z0, (int)Wz, ROWS * pass)));
         dim3 g(P.nA, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
-        STAGE(tm, 4, s, (mixed_gather_kernel<Ti, T><<<g, 256, 0, s>>>(ma, B->view, Z, dst, z0, (int)Wz)));
+        STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0, (int)Wz)));
     }
     return BSIM_OK;
 }
@@ -1161,7 +1271,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                                                            tcGrow, s));
                 if (rc != BSIM_OK) return rc;
                 dim3 g(P.nA, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
-                STAGE(tm, 4, s, (mixed_gather_kernel<Ti, T><<<g, 256, 0, s>>>(ma, B->view, Z, dst, z0, (int)Wz)));
+                STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0, (int)Wz)));
             }
             return BSIM_OK;
         }
@@ -1179,9 +1289,10 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                 const size_t Wz = z.w;
                 for (int z0 = c0; z0 < c1; z0 += (int)Wz) {
                     for (int pass = 0; pass < passes; ++pass)
-                        STAGE(tm, 3, s, (kern<<<P.nA, 512, smem, s>>>(ma, P.d_astr, ct, Z, z0, (int)Wz, 64 * pass)));
+                        STAGE(tm, 3, s, (launch_chained(kern, P.nA, 512, smem, s, ma, P.d_astr, ct, Z, z0, (int)Wz,
+                                                       64 * pass)));
                     dim3 g(P.nA, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
-                    STAGE(tm, 4, s, (mixed_gather_kernel<Ti, T><<<g, 256, 0, s>>>(ma, B->view, Z, dst, z0, (int)Wz)));
+                    STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0, (int)Wz)));
                 }
                 return BSIM_OK;
             }
@@ -1241,9 +1352,9 @@ static int launch_ri(const RISide &R, const T *in, int ld_in, double *out, int l
             const size_t sm = ri_dmma_smem(R.nU);
             BSIM_CUDA(cudaFuncSetAttribute(ri_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             for (int z0 = c0; z0 < c1; z0 += (int)Wz) {
-                STAGE(tm, 7, s, (ri_dmma_kernel<<<R.nM, 512, sm, s>>>(ra, in, Z, z0, (int)Wz)));
+                STAGE(tm, 7, s, (launch_chained(ri_dmma_kernel, R.nM, 512, sm, s, ra, in, Z, z0, (int)Wz)));
                 dim3 g(nrows, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
-                STAGE(tm, 8, s, (ri_gather_kernel<T><<<g, 256, 0, s>>>(ra, R.gath, Z, out, ld_out, z0, (int)Wz)));
+                STAGE(tm, 8, s, (launch_chained(ri_gather_kernel<T>, g, 256, 0, s, ra, R.gath, Z, out, ld_out, z0, (int)Wz)));
             }
             return BSIM_OK;
         }
@@ -1260,7 +1371,7 @@ static int launch_ri(const RISide &R, const T *in, int ld_in, double *out, int l
         }
         if (!tc) STAGE(tm, 7, s, (ri_gemm_kernel<T, EPT><<<R.nM, NT, smem, s>>>(ra, in, Z, z0, (int)Wz)));
         dim3 g(nrows, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
-        STAGE(tm, 8, s, (ri_gather_kernel<T><<<g, 256, 0, s>>>(ra, R.gath, Z, out, ld_out, z0, (int)Wz)));
+        STAGE(tm, 8, s, (launch_chained(ri_gather_kernel<T>, g, 256, 0, s, ra, R.gath, Z, out, ld_out, z0, (int)Wz)));
     }
     return BSIM_OK;
 }
@@ -1281,21 +1392,19 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     dim3 tgrid((nB + 31) / 32, (nA + 31) / 32), tblk(32, 8);
     auto frame = [&](T *ct, T *ctT) {
         if (src32)
-            frame_transpose_kernel<Ti, float, T><<<tgrid, tblk, 0, s>>>(nA, nB, P.ldA, P.ldB, P.d_bstr, P.d_Ka, src32,
-                                                                         ct, ctT);
+            launch_chained(frame_transpose_kernel<Ti, float, T>, tgrid, tblk, 0, s, nA, nB, P.ldA, P.ldB, P.d_bstr,
+                           P.d_Ka, src32, ct, ctT);
         else
-            frame_transpose_kernel<Ti, double, T><<<tgrid, tblk, 0, s>>>(nA, nB, P.ldA, P.ldB, P.d_bstr, P.d_Ka, src,
-                                                                          ct, ctT);
+            launch_chained(frame_transpose_kernel<Ti, double, T>, tgrid, tblk, 0, s, nA, nB, P.ldA, P.ldB, P.d_bstr,
+                           P.d_Ka, src, ct, ctT);
     };
     // FP64: 16 warps of DMMA 8x8 tiles; FP32: 8 warps of 8 x 4 f32x2 register tiles
     constexpr int kEPT = sizeof(T) == 8 ? 4 : 8;
     // ---- alpha side: c~ in `in`, results into dst; tT's buffer is free for Z ----
     STAGE(tm, 0, s, frame(in, nullptr));
-    {   // pure alpha + diagonal -> dst (the frame's s~)
-        dim3 g(nA, (c1 - c0 + kRowChunk - 1) / kRowChunk);
-        STAGE(tm, 1, s, (pure_rows_kernel<T><<<g, 256, 0, s>>>(0, c0, c1, P.ldA, P.csrA, in, dst, nB,
-                                                               P.rank_d ? P.d_PAd : nullptr, P.d_PBdT, P.rank_d)));
-    }
+    // pure alpha + diagonal -> dst (the frame's s~)
+    STAGE(tm, 1, s, launch_pure<T>(0, nA, c0, c1, P.ldA, P.csrA, in, dst, nB, P.rank_d ? P.d_PAd : nullptr, P.d_PBdT,
+                                   P.rank_d, s));
     if (P.riA.on) {   // same-spin alpha doubles through intermediate strings -> dst
         rc = launch_ri<T, kEPT>(P.riA, in, P.ldA, dst, nB, nA, c0, c1, &S.Z, &S.z_n, S.tT, S.tT_n, s, tm);
         if (rc != BSIM_OK) return rc;
@@ -1316,18 +1425,15 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     //      intermediates when the whole sigma is computed, else through the rows) ----
     STAGE(tm, 0, s, frame(nullptr, in));
     const bool ri_b = P.riB.on && c0 == 0 && c1 == nB;
-    {
-        dim3 g(c1 - c0, (nA + kRowChunk - 1) / kRowChunk);
-        STAGE(tm, 2, s, (pure_rows_kernel<T><<<g, 256, 0, s>>>(c0, 0, nA, P.ldB, ri_b ? P.csrBri : P.csrB, in, tT,
-                                                               P.ldB, nullptr, nullptr, 0)));
-    }
+    STAGE(tm, 2, s, launch_pure<T>(c0, c1, 0, nA, P.ldB, ri_b ? P.csrBri : P.csrB, in, tT, P.ldB, nullptr, nullptr, 0, s));
     if (ri_b) {
         rc = launch_ri<T, kEPT>(P.riB, in, P.ldB, tT, P.ldB, nB, 0, nA, &S.Z, &S.z_n, nullptr, 0, s, tm);
         if (rc != BSIM_OK) return rc;
     }
     // ---- final combine ----
     dim3 fgrid((c1 - c0 + 31) / 32, (nA + 31) / 32);
-    STAGE(tm, 5, s, (final_kernel<Ti><<<fgrid, tblk, 0, s>>>(nA, nB, P.ldB, c0, c1, P.d_bstr, P.d_Ka, tT, dst)));
+    STAGE(tm, 5, s, (launch_chained(final_kernel<Ti>, fgrid, tblk, 0, s, nA, nB, P.ldB, c0, c1, P.d_bstr, P.d_Ka, tT,
+                                     dst)));
     BSIM_CUDA(cudaGetLastError());
     return BSIM_OK;
 }

@@ -1,0 +1,32 @@
+"""Pure-spin rows with the entries divided among warps (small bases) and one CTA per 1024 columns (larger ones): both
+sides of the line, columns that end inside a tile, column ranges, FP64 and FP32 bulk, against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import dev
+
+pytestmark = pytest.mark.gpu
+
+
+# rows x column tiles of the row kernel: 2, 70, 462, 495 (below the line of 512), 715 and 792 (above it)
+@pytest.mark.parametrize("norb,na,nb", [(2, 1, 1), (8, 4, 4), (11, 5, 5), (12, 4, 2), (13, 4, 3), (12, 5, 5)])
+def test_matches_oracle(cuda, oracle, norb, na, nb):
+    from binsim_b200 import cuotf, network as nw
+    net = nw.hamiltonian_network(norb, seed=7, native=True)
+    B = cuotf.CuBasis(norb, na, nb)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+    x = np.random.default_rng(norb).normal(size=B.dim)
+    x /= np.linalg.norm(x)
+    ref = oracle.hvec(oracle.basis(norb, na, nb), oracle.network(net), x)
+    scale = np.abs(ref).max()
+    y = cuda.full((B.dim,), float("nan"), dtype=cuda.float64, device="cuda")
+    f.hvec(dev(cuda, x), y)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 1e-12 * scale
+    # FP32 bulk: sums of at most a few hundred products of FP32 factors, each rounded at 2^-24
+    f.hvec_mixed(dev(cuda, x), y)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 1e-5 * scale
+    # repeated calls give the same bits: the warps' sums are added in a fixed order
+    z = cuda.empty_like(y)
+    f.hvec(dev(cuda, x), y)
+    f.hvec(dev(cuda, x), z)
+    assert bool((y == z).all())

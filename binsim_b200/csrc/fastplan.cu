@@ -107,7 +107,7 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     }
     if (norb > 63) { P->why = "norb > 63"; return BSIM_OK; }
     P->norb = norb; P->nA = nA; P->nB = nB; P->nelA = nelA; P->nelB = nelB;
-    P->ldA = (nB + 7) & ~7;
+    P->ldA = (nB + 8) & ~7;
     P->ldB = (nA + 7) & ~7;
     P->ldG = (nB + kMixCols - 1) / kMixCols * kMixCols;
     P->Ka.resize(nA);
@@ -458,6 +458,26 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
             }
     }
 
+    // the same as byte offsets into rows of 8-byte words, by column, F to whole slices
+    const int nFp = (P->nF + 31) & ~31;
+    std::vector<unsigned> goff((size_t)P->ldG * nFp, (unsigned)nB * 8u);
+    for (int f = 0; f < P->nF; ++f)
+        for (int b = 0; b < nB; ++b) {
+            const int g = gidx[(size_t)f * P->ldG + b];
+            if (g >= 0) goff[(size_t)b * nFp + f] = (unsigned)(g >> 1) * 8u | (unsigned)(g & 1) << 31;
+        }
+    std::vector<int> lexp(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
+    for (int e = 0; e < P->nE; ++e) {
+        double m = 0.0;
+        bool bad = false;
+        for (int f = 0; f < P->nF; ++f) {
+            const double v = std::fabs(P->Lam[(size_t)e * P->nF + f]);
+            bad = bad || !std::isfinite(v);
+            m = std::max(m, v);
+        }
+        lexp[e] = bad ? 0x7fffffff : m > 0.0 ? std::ilogb(m) + 1 : -2000;
+    }
+
     // ---- intermediate-string tables ----------------------------------------------
     struct RIHost {
         int nM = 0, nU = 0, npr = 0;
@@ -530,6 +550,7 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     auto bytes = [](size_t n, size_t sz) { return ((std::max<size_t>(n, 1) * sz) + 255) & ~size_t(255); };
     size_t tot = bytes(nA, sizeof(Ti)) + bytes(nB, sizeof(Ti)) + bytes(nA, 8) + bytes(PAd.size(), 8) +
                  bytes(PBd.size(), 8) + 2 * bytes(P->nE, 8) + 2 * bytes(P->Lam.size(), 8) + bytes(gidx.size(), 4) +
+                 bytes(goff.size(), 4) + bytes(lexp.size(), 4) +
                  bytes(P->residual.size(), 4) + bytes(P->residual.size() + 1, 16);
     for (int li = 0; li < 3; ++li)
         tot += 2 * bytes(csr[li].cptr.size(), 8) + bytes(csr[li].cent.size(), sizeof(CEnt)) +
@@ -557,6 +578,8 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     std::vector<float> lam32(P->Lam.begin(), P->Lam.end());
     P->d_Lam32 = put(lam32);
     P->d_gidx = put(gidx);
+    P->d_goff = put(goff);
+    P->d_lexp = put(lexp);
     for (int li = 0; li < 3; ++li) {
         CSRHost &C = csr[li];
         if (li == 2 && !ri_on[1]) continue;

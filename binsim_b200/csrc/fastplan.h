@@ -81,7 +81,8 @@ struct FastPlan {
     const void *basis = nullptr;
     i64 basis_dim = -1;
     int norb = 0, nA = 0, nB = 0, nelA = 0, nelB = 0;
-    // padded row strides: ldA for rows of c~ (alpha rows, beta columns), ldB for
+    // padded row strides: ldA for rows of c~ (alpha rows, beta columns; at least one
+    // padding column, a zero that the gather tables can name), ldB for
     // rows of c~^T and of the beta-side result, ldG for the gather-index table
     int ldA = 0, ldB = 0, ldG = 0;
     // frame
@@ -111,6 +112,8 @@ struct FastPlan {
     const float *d_Lam32 = nullptr;
     const double *d_PBdT = nullptr;    // [rank_d x ldA] beta diagonal factors, transposed
     const int *d_gidx = nullptr;       // [nF x ldG] (rank(b^F) << 1 | sign) or -1
+    const unsigned *d_goff = nullptr;  // the same as byte offsets, by column (MixedArgs)
+    const int *d_lexp = nullptr;       // [nE] exponent above a row of Lam
     const int *d_resid = nullptr;      // residual group plan (for the generic kernel)
     const int4 *d_resid_chunks = nullptr;
     int n_resid_chunks = 0;
@@ -148,7 +151,7 @@ inline size_t mixed_smem_bytes(int nB, int nF, size_t elem, bool stream, bool gr
 {
     const size_t lam_rows = stream ? 32 : (((size_t)nF + 7) & ~size_t(7));
     const size_t ls = rows > 64 ? (size_t)rows : gemm_ls(elem);
-    return (grow ? 0 : (((size_t)nB + 7) & ~size_t(7)) * elem) + lam_rows * ls * elem +
+    return (grow ? 0 : (((size_t)nB + 8) & ~size_t(7)) * elem) + lam_rows * ls * elem +
            32 * gemm_xs(elem) * elem + 2 * kMaxConn * 4;
 }
 

@@ -12,6 +12,10 @@ struct MixedArgs {
     const u64 *Emask, *mA;
     const void *Lam;        // T [nE x nF]
     const int *gidx;        // [nF x ldG]: (rank(b^F) << 1 | sign) or -1
+    // split products: byte offset of b^F in a row of 8-byte words | sign << 31, the
+    // padding column (zero) where there is none; [ldG x (nF rounded up to 32)]
+    const unsigned *goff;
+    const int *lexp;        // [nE] exponent above a row of Lam
 };
 
 // Layout of the GEMM outputs Z (a window of W columns, W a multiple of 128):
@@ -74,5 +78,18 @@ bool ri_tc_supported(int nU);
 size_t ri_tc_smem(int nU);
 int ri_gemm_tc(const RIArgs &ra, const float *in, float *Z, int z0, int W, cudaStream_t s);
 int mixed_tc_timeouts(int *count, bool reset);
+
+// The mixed product of the FP64 sigma as split products on the tensor cores
+// (sigma_split.cu), up to kSplitRows output rows per pass (from jbase).  It reads the
+// rows of c~ as fixed-point words with one exponent per row, which rows_to_fixed makes
+// in place.
+constexpr int kSplitRows = 64;
+// output rows per pass, 0: no kernel for the shape
+int mixed_split_rows(int nF, int M);
+int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s);
+template <typename Ti>
+int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, const double *ct, const int *rexp, double *Z, int z0, int W,
+                     int jbase, int rows, cudaStream_t s);
+int split_timeouts(int *count, bool reset);
 
 }  // namespace bsim

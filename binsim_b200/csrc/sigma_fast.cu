@@ -1235,8 +1235,41 @@ static MixedTc mixed_tc_mode()
     return MixedTc::automatic;
 }
 
+// BSIM_SIGMA_SPLIT (read on every call: tests compare the two): 0 sends the FP64 mixed
+// product to the DMMA kernels, 1 to the split products at every size they fit.
+// BSIM_MIXED_DMMA and BSIM_MIXED_ROW_SMEM choose between the DMMA kernels, so they too
+// send it there.
+enum class Split { automatic, never, always };
+static Split split_mode()
+{
+    if (const char *e = getenv("BSIM_SIGMA_SPLIT")) {
+        if (e[0] == '0') return Split::never;
+        if (e[0] == '1') return Split::always;
+    }
+    return getenv("BSIM_MIXED_DMMA") || getenv("BSIM_MIXED_ROW_SMEM") ? Split::never : Split::automatic;
+}
+
+// Output rows per pass of the split mixed product, 0: the DMMA kernels.  The split
+// kernel works on chunks of 128 columns and needs two to keep its warps busy, and its
+// rows_to_fixed and staging cost ~8 us (both kernels, us, DMMA / split): one chunk
+// loses, 312 / 353 at 14o 7+2 (91 columns), 908 / 1039 at 16o 6+2 (120); so do small
+// products, 12.4 / 21.1 at 10o 3+3, 29.7 / 35.4 at 10o 5+5 (2.9 M rows x columns x F);
+// 41.2 / 39.4 at 12o 3+3 (3.2 M), 72 / 48 at 18o 2+2 (3.6 M, 153 columns), 101 / 85 at
+// 11o 5+5 (11.7 M), 1295 / 837 at 20o 3+3.  By the whole basis, not by the call's
+// columns: column bands of one sigma give the same bits however they are cut.
+constexpr int kSplitMinCols = 129;
+constexpr double kSplitMinWork = 3.1e6;
+template <typename Ti>
+static int mixed_split(const FastPlan<Ti> &P)
+{
+    const Split mode = split_mode();
+    if (mode == Split::never) return 0;
+    if (mode == Split::automatic && (P.nB < kSplitMinCols || (double)P.nA * P.nB * P.nF < kSplitMinWork)) return 0;
+    return mixed_split_rows(P.nF, P.M);
+}
+
 template <typename Ti, typename T, int EPT>
-static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> &S, const T *ct, double *dst,
+static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> &S, T *ct, double *dst,
                         int c0, int c1, cudaStream_t s, StageTimer *tm)
 {
     const size_t per_col = (size_t)P.nA * P.M * sizeof(T);
@@ -1244,7 +1277,26 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
     int rc = z_slot(&S.Z, &S.z_n, S.tT, S.tT_n, per_col, c1 - c0, &z);
     if (rc != BSIM_OK) return rc;
     MixedArgs ma{P.nA, P.nB, P.nE, P.nF, P.M, P.ldA, P.ldG, c1, P.d_Emask, P.d_mA,
-                 sizeof(T) == 8 ? (const void *)P.d_Lam : (const void *)P.d_Lam32, P.d_gidx};
+                 sizeof(T) == 8 ? (const void *)P.d_Lam : (const void *)P.d_Lam32, P.d_gidx, P.d_goff, P.d_lexp};
+    if constexpr (sizeof(T) == 8) {
+        const int rows = mixed_split(P);
+        if (rows > 0) {   // split products; nothing reads c~ in floating point after this
+            int *rexp = reinterpret_cast<int *>(ct + (size_t)P.nA * P.ldA);   // behind the rows (run_fast)
+            double *Z = static_cast<double *>(z.p);
+            STAGE(tm, 3, s, rc = rows_to_fixed(ct, P.nA, P.ldA, rexp, s));
+            if (rc != BSIM_OK) return rc;
+            for (int z0 = c0; z0 < c1; z0 += (int)z.w) {
+                for (int jb = 0; jb < P.M; jb += rows) {
+                    STAGE(tm, 3, s, rc = mixed_gemm_split<Ti>(ma, P.d_astr, ct, rexp, Z, z0, (int)z.w, jb, rows, s));
+                    if (rc != BSIM_OK) return rc;
+                }
+                dim3 g(P.nA, (unsigned)((std::min<size_t>(z.w, c1 - z0) + kRowChunk - 1) / kRowChunk));
+                STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0,
+                                                (int)z.w)));
+            }
+            return BSIM_OK;
+        }
+    }
     if constexpr (sizeof(T) == 4) {
         // FP32 bulk: the tensor-core (TF32 x 3) kernel, with the source row on chip
         // where it fits, else gathered from global memory (80 excitations per pass
@@ -1384,12 +1436,13 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     FastScratch<Ti> &S = st->scratch;
     const int nA = P.nA, nB = P.nB;
     int rc;
-    const size_t in_bytes = std::max((size_t)nA * P.ldA, (size_t)nB * P.ldB) * sizeof(T);
+    // c~ (behind it the exponents of its rows as fixed-point numbers), later c~^T
+    const size_t in_bytes = std::max((size_t)nA * P.ldA * sizeof(T) + (size_t)nA * sizeof(int), (size_t)nB * P.ldB * sizeof(T));
     if ((rc = ensure(&S.in, &S.in_n, in_bytes)) != BSIM_OK) return rc;
     if ((rc = ensure(&S.tT, &S.tT_n, (size_t)nB * P.ldB * sizeof(double))) != BSIM_OK) return rc;
     T *in = static_cast<T *>(S.in);
     double *tT = static_cast<double *>(S.tT);
-    dim3 tgrid((nB + 31) / 32, (nA + 31) / 32), tblk(32, 8);
+    dim3 tgrid((P.ldA + 31) / 32, (P.ldB + 31) / 32), tblk(32, 8);   // the padding columns too
     auto frame = [&](T *ct, T *ctT) {
         if (src32)
             launch_chained(frame_transpose_kernel<Ti, float, T>, tgrid, tblk, 0, s, nA, nB, P.ldA, P.ldB, P.d_bstr,

@@ -46,6 +46,7 @@
 // frees its tensor memory before it exits.
 #include "mixed.cuh"
 #include "ops.h"
+#include "tc.cuh"
 
 #include <cstdlib>
 
@@ -61,10 +62,6 @@ constexpr int kMixKS = 48;                // F rows per A slice of the mixed pro
 constexpr int kMixKSGrow = 40;            // the same, row read from global memory
 constexpr int kMixStages = 2;             // its A stages
 constexpr int kRiStages = 2, kRiRing = 4; // the intermediate product's A stages and copy-ring slots
-constexpr unsigned long long kTcWaitNs = 20000000ull;   // a wait gives up after 20 ms
-constexpr long kTcSpinCap = 1L << 26;                   // and after this many rounds in any case
-constexpr unsigned kTcSuspendNs = 20000;                // longest sleep in one test of a phase
-constexpr uint32_t kCoreBytes = 128;      // one core matrix: 8 rows x 16 bytes (4 TF32)
 
 // two N-column accumulators, allocated as a power of 2 of at least 32 columns
 template <int N>
@@ -75,16 +72,12 @@ template <int N>
 constexpr uint32_t idesc_tf32() { return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) |
                                          ((uint32_t)(kTcM >> 4) << 24); }
 
-__device__ int g_tc_timeouts;   // waits that gave up
-__device__ int g_tc_abort;      // set with the first of them: later CTAs return at once
-
 // Shared-memory layout (bytes from the dynamic base, 128-byte aligned pieces).
 struct TcLayout {
     uint32_t srow, bh, bl, ah, al, abytes, tab, bars, tmem, total;
     int kp8;        // K rounded up to the MMA's K step (8)
     uint32_t sbo_b; // byte stride between 8-row groups of B (all K chunks of a group)
 };
-__host__ __device__ inline uint32_t align128(uint32_t x) { return (x + 127u) & ~127u; }
 // srow_bytes: the source row staged on chip (0 when it is not); S: A stages of
 // KS rows (hi and lo parts); tab_bytes: the CTA's index tables
 __host__ __device__ inline TcLayout tc_layout(uint32_t srow_bytes, int K, int N, int KS, int S, uint32_t tab_bytes)
@@ -126,90 +119,12 @@ __host__ __device__ inline TcLayout ri_layout(int K)
                      ri_raw_off() + (uint32_t)(kRiRing * KS * kTcM * 4));
 }
 
-__device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t a)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(a) : "memory");
-}
-// One test of the phase; the thread may sleep in it (up to kTcSuspendNs) until
-// the phase completes, so a waiting warp takes no issue slots from the others.
-__device__ __forceinline__ bool mbar_try(uint32_t a, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
-                 "selp.b32 %0, 1, 0, P1;\n\t}"
-                 : "=r"(ok)
-                 : "r"(a), "r"(parity), "n"(kTcSuspendNs)
-                 : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait for the phase of the given parity; false when the CTA aborts
-// (its own wait gave up, another wait of the CTA did, or another CTA's did).
-// The flags and the clock are read after each test that came back without the
-// phase, i.e. at most once per suspend period.
-__device__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int *abort_flag)
-{
-    if (mbar_try(a, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (long i = 1; i < kTcSpinCap; ++i) {
-        if (mbar_try(a, parity)) return true;
-        if (*abort_flag) return false;
-        if (*(volatile int *)&g_tc_abort) { *abort_flag = 1; return false; }
-        if (global_ns() - t0 > kTcWaitNs) break;
-    }
-    *abort_flag = 1;
-    atomicExch(&g_tc_abort, 1);
-    atomicAdd(&g_tc_timeouts, 1);
-    return false;
-}
-
-// Bounded wait that ignores the abort flags: the wait for this CTA's own MMAs
-// before its tensor memory is freed.
-__device__ void mbar_wait_drain(uint32_t a, uint32_t parity)
-{
-    const unsigned long long t0 = global_ns();
-    for (long i = 0; i < kTcSpinCap; ++i) {
-        if (mbar_try(a, parity)) return;
-        if (global_ns() - t0 > kTcWaitNs) break;
-    }
-    atomicExch(&g_tc_abort, 1);
-    atomicAdd(&g_tc_timeouts, 1);
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Shared-memory matrix descriptor: no swizzle (canonical K-major core matrices),
-// leading byte offset = next K chunk, stride byte offset = next 8-row group,
-// descriptor version 1 (bits 46-47).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
                                           uint32_t accumulate)
 {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                  "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                  : "memory");
 }
 // 16 consecutive FP32 columns of this thread's TMEM lane, waited for.
@@ -793,8 +708,10 @@ int mixed_tc_timeouts(int *count, bool reset)
         BSIM_CUDA(cudaMemcpyToSymbol(g_tc_timeouts, &z, sizeof(int)));
         BSIM_CUDA(cudaMemcpyToSymbol(g_tc_abort, &z, sizeof(int)));
     }
-    *count = h;
-    return BSIM_OK;
+    int h8 = 0;
+    const int st = split_timeouts(&h8, reset);
+    *count = h + h8;
+    return st;
 }
 
 template int mixed_gemm_tc<unsigned>(const MixedArgs &, const unsigned *, const float *, float *, int, int, int, int,

@@ -269,13 +269,16 @@ pure_split_kernel(int row_begin, int col_begin, int ncols, int ld_in, const Side
     }
 }
 
+// By the whole side (rows x columns), not by the call's band: column bands of one
+// sigma give the same bits however they are cut.
+static bool few_rows(int rows, int cols) { return (i64)rows * ((cols + kRowChunk - 1) / kRowChunk) < kSplitCtas; }
+
 template <typename T>
-static void launch_pure(int row0, int row1, int c0, int c1, int ld_in, const SideCSR &L, const T *in, double *out,
-                        int ld_out, const double *PAd, const double *PBdT, int rank_d, cudaStream_t s)
+static void launch_pure(bool few, int row0, int row1, int c0, int c1, int ld_in, const SideCSR &L, const T *in,
+                        double *out, int ld_out, const double *PAd, const double *PBdT, int rank_d, cudaStream_t s)
 {
-    const i64 ctas = (i64)(row1 - row0) * ((c1 - c0 + kRowChunk - 1) / kRowChunk);
     if (row1 <= row0 || c1 <= c0) return;
-    if (ctas < kSplitCtas) {
+    if (few) {
         dim3 g(row1 - row0, (c1 - c0 + kSplitCols - 1) / kSplitCols);
         launch_chained(pure_split_kernel<T>, g, 256, 0, s, row0, c0, c1, ld_in, L, in, out, ld_out, PAd, PBdT, rank_d);
     } else {
@@ -1456,8 +1459,8 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     // ---- alpha side: c~ in `in`, results into dst; tT's buffer is free for Z ----
     STAGE(tm, 0, s, frame(in, nullptr));
     // pure alpha + diagonal -> dst (the frame's s~)
-    STAGE(tm, 1, s, launch_pure<T>(0, nA, c0, c1, P.ldA, P.csrA, in, dst, nB, P.rank_d ? P.d_PAd : nullptr, P.d_PBdT,
-                                   P.rank_d, s));
+    STAGE(tm, 1, s, launch_pure<T>(few_rows(nA, nB), 0, nA, c0, c1, P.ldA, P.csrA, in, dst, nB,
+                                   P.rank_d ? P.d_PAd : nullptr, P.d_PBdT, P.rank_d, s));
     if (P.riA.on) {   // same-spin alpha doubles through intermediate strings -> dst
         rc = launch_ri<T, kEPT>(P.riA, in, P.ldA, dst, nB, nA, c0, c1, &S.Z, &S.z_n, S.tT, S.tT_n, s, tm);
         if (rc != BSIM_OK) return rc;
@@ -1478,7 +1481,8 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     //      intermediates when the whole sigma is computed, else through the rows) ----
     STAGE(tm, 0, s, frame(nullptr, in));
     const bool ri_b = P.riB.on && c0 == 0 && c1 == nB;
-    STAGE(tm, 2, s, launch_pure<T>(c0, c1, 0, nA, P.ldB, ri_b ? P.csrBri : P.csrB, in, tT, P.ldB, nullptr, nullptr, 0, s));
+    STAGE(tm, 2, s, launch_pure<T>(few_rows(nB, nA), c0, c1, 0, nA, P.ldB, ri_b ? P.csrBri : P.csrB, in, tT, P.ldB, nullptr,
+                                   nullptr, 0, s));
     if (ri_b) {
         rc = launch_ri<T, kEPT>(P.riB, in, P.ldB, tT, P.ldB, nB, 0, nA, &S.Z, &S.z_n, nullptr, 0, s, tm);
         if (rc != BSIM_OK) return rc;

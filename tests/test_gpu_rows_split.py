@@ -30,3 +30,21 @@ def test_matches_oracle(cuda, oracle, norb, na, nb):
     f.hvec(dev(cuda, x), y)
     f.hvec(dev(cuda, x), z)
     assert bool((y == z).all())
+
+
+@pytest.mark.parametrize("norb,na,nb", [(12, 5, 5), (13, 3, 6)])
+def test_column_bands_give_the_same_bits(cuda, norb, na, nb):
+    """Bands whose own rows fall below the line, cut in two ways: the kernel is chosen by the whole side."""
+    import math
+    from binsim_b200 import cuotf, network as nw
+    B = cuotf.CuBasis(norb, na, nb)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(nw.hamiltonian_network(norb, seed=7, native=True)))
+    x = dev(cuda, np.random.default_rng(norb).normal(size=B.dim))
+    nB = math.comb(norb, nb)
+    out = []
+    for cuts in ((0, 128, nB), (0, 640, nB)):
+        y = cuda.empty_like(x)
+        for lo, hi in zip(cuts, cuts[1:]):
+            f.hvec_cols(x, y, lo, hi)
+        out.append(y)
+    assert cuda.equal(out[0], out[1])

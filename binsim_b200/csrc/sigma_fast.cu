@@ -1240,8 +1240,7 @@ static MixedTc mixed_tc_mode()
 
 // BSIM_SIGMA_SPLIT (read on every call: tests compare the two): 0 sends the FP64 mixed
 // product to the DMMA kernels, 1 to the split products at every size they fit.
-// BSIM_MIXED_DMMA and BSIM_MIXED_ROW_SMEM choose between the DMMA kernels, so they too
-// send it there.
+// BSIM_MIXED_DMMA chooses between the DMMA kernels, so it too sends it there.
 enum class Split { automatic, never, always };
 static Split split_mode()
 {
@@ -1249,7 +1248,7 @@ static Split split_mode()
         if (e[0] == '0') return Split::never;
         if (e[0] == '1') return Split::always;
     }
-    return getenv("BSIM_MIXED_DMMA") || getenv("BSIM_MIXED_ROW_SMEM") ? Split::never : Split::automatic;
+    return getenv("BSIM_MIXED_DMMA") ? Split::never : Split::automatic;
 }
 
 // Output rows per pass of the split mixed product, 0: the DMMA kernels.  The split

@@ -34,13 +34,19 @@ def test_matches_oracle_and_dmma(cuda, oracle, monkeypatch, norb, na, nb):
     z = cuda.empty_like(y)
     f.hvec(dev(cuda, x), z)
     scale = np.abs(ref).max()
+    # the DMMA kernel with the source row in global memory: the same bits
+    monkeypatch.setenv("BSIM_MIXED_ROW_SMEM", "1")
+    w = cuda.empty_like(y)
+    f.hvec(dev(cuda, x), w)
+    monkeypatch.delenv("BSIM_MIXED_ROW_SMEM")
+    assert cuda.equal(w, z)
     assert np.abs(y.cpu().numpy() - ref).max() <= 1e-12 * scale
     # both round their sums at 2^-53 of terms no larger than the largest element of H x
     assert float((y - z).abs().max()) <= 1e-13 * scale
     # in column bands (their starts multiples of 128; the beta doubles take another route)
     monkeypatch.setenv("BSIM_SIGMA_SPLIT", "1")
     nB = math.comb(norb, nb)
-    w = cuda.full_like(y, float("nan"))
+    w.fill_(float("nan"))
     for lo, hi in ((0, min(nB, 128)), (128, nB)):
         if lo < hi:
             f.hvec_cols(dev(cuda, x), w, lo, hi)

@@ -30,7 +30,8 @@
 
 namespace bsim {
 
-constexpr int kRowChunk = 1024;        // columns per CTA in the row kernels (256 threads x 4)
+constexpr int kRowChunk = 1024;        // columns per CTA in the gather kernels (256 threads x 4)
+template <typename T> constexpr int kRowThreads = sizeof(T) == 8 ? 256 : 384;   // of a CTA of pure_rows_kernel
 constexpr int kSplitCtas = 512;        // below this many CTAs of the row kernel: pure_split_kernel (measured there)
 
 template <typename T> struct Vec2;
@@ -80,19 +81,25 @@ __global__ void frame_transpose_kernel(int nA, int nB, int ldA, int ldB, const T
 }
 
 // ---- 2/3. pure groups of one spin: row AXPY over the precomputed row lists -----------
-// One CTA per (row, 1024-column chunk) of rows row_begin.. and columns
-// [col_begin, ncols); each thread owns 4 consecutive columns.
+// One CTA per (row, chunk of columns) of rows row_begin.. and columns
+// [col_begin, ncols); each thread owns 4 consecutive columns.  The chunks are cut
+// evenly, at most kRowThreads threads each: a last chunk of a few columns walks the
+// whole row's entries for them.  Alpha + beta rows, ms, against chunks of 1024 columns:
+// FP64 1.12 -> 0.99 at 20o 3+3 (1140 columns), 0.40 -> 0.375 at 13o 7+5; FP32
+// 0.595 -> 0.484 at 20o 3+3, 1.42 -> 1.31 at 14o 7+7, 26.3 -> 24.6 at 16o 8+8.  FP32
+// takes up to 384 threads (256: 0.56 at 20o, 1.47 at 14o); FP64, whose tables fill L1
+// sooner, 256 (384: 40.6 ms at 16o against 38.9).
 // Constant-factor entries accumulate in T over batches of 64 entries, then in
 // FP64; table entries and the diagonal are FP64 throughout.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRowThreads<T>)
 pure_rows_kernel(int row_begin, int col_begin, int ncols, int ld_in, const SideCSR L, const T *__restrict__ in,
                  double *__restrict__ out, int ld_out, const double *__restrict__ PAd, const double *__restrict__ PBdT,
                  int rank_d)
 {
     chain_wait();
     const int row = row_begin + blockIdx.x;
-    const int c = col_begin + blockIdx.y * kRowChunk + 4 * threadIdx.x;
+    const int c = col_begin + 4 * (int)(blockIdx.y * blockDim.x + threadIdx.x);
     if (c >= ncols) return;
     const T *in_c = in + c;
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
@@ -282,8 +289,10 @@ static void launch_pure(bool few, int row0, int row1, int c0, int c1, int ld_in,
         dim3 g(row1 - row0, (c1 - c0 + kSplitCols - 1) / kSplitCols);
         launch_chained(pure_split_kernel<T>, g, 256, 0, s, row0, c0, c1, ld_in, L, in, out, ld_out, PAd, PBdT, rank_d);
     } else {
-        dim3 g(row1 - row0, (c1 - c0 + kRowChunk - 1) / kRowChunk);
-        launch_chained(pure_rows_kernel<T>, g, 256, 0, s, row0, c0, c1, ld_in, L, in, out, ld_out, PAd, PBdT, rank_d);
+        const int quads = (c1 - c0 + 3) / 4, chunks = (quads + kRowThreads<T> - 1) / kRowThreads<T>;
+        const int threads = ((quads + chunks - 1) / chunks + 31) / 32 * 32;
+        launch_chained(pure_rows_kernel<T>, dim3(row1 - row0, chunks), threads, 0, s, row0, c0, c1, ld_in, L, in, out,
+                       ld_out, PAd, PBdT, rank_d);
     }
 }
 

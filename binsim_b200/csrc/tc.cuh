@@ -57,8 +57,8 @@ __device__ __forceinline__ unsigned long long global_ns()
 
 // Bounded wait for the phase of the given parity; false when the CTA aborts
 // (its own wait gave up, another wait of the CTA did, or another CTA's did).
-// The flags and the clock are read after each test that came back without the
-// phase, i.e. at most once per suspend period.
+// The flags and the clock are read after every kTcCheck tests that came back without
+// the phase.
 __device__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int *abort_flag)
 {
     if (mbar_try(a, parity)) return true;

@@ -1,5 +1,5 @@
-"""Pure-spin rows with the entries divided among warps (small bases) and one CTA per 1024 columns (larger ones): both
-sides of the line, columns that end inside a tile, column ranges, FP64 and FP32 bulk, against the oracle."""
+"""Pure-spin rows with the entries divided among warps (small bases) and one CTA per even chunk of columns (larger
+ones): both sides of the line, columns that end inside a tile, FP64 and FP32 bulk, against the oracle."""
 import numpy as np
 import pytest
 
@@ -8,8 +8,9 @@ from conftest import dev
 pytestmark = pytest.mark.gpu
 
 
-# rows x column tiles of the row kernel: 2, 70, 462, 495 (below the line of 512), 715 and 792 (above it)
-@pytest.mark.parametrize("norb,na,nb", [(2, 1, 1), (8, 4, 4), (11, 5, 5), (12, 4, 2), (13, 4, 3), (12, 5, 5)])
+# rows x 1024-column tiles: 2, 70, 462, 495 (below the line of 512), 715 and 792 (above it), 715 x 2: rows of 1287
+# columns, two chunks of 161 quads in FP64 and one of 322 in FP32
+@pytest.mark.parametrize("norb,na,nb", [(2, 1, 1), (8, 4, 4), (11, 5, 5), (12, 4, 2), (13, 4, 3), (12, 5, 5), (13, 4, 5)])
 def test_matches_oracle(cuda, oracle, norb, na, nb):
     from binsim_b200 import cuotf, network as nw
     net = nw.hamiltonian_network(norb, seed=7, native=True)

@@ -41,6 +41,7 @@ constexpr unsigned kPoolDensityMagic = 0xB5B1D7A1u;
 constexpr int kTK = 32, kTM = 64, kTN = 128;     // K slice, output tile
 constexpr int kLS = kTM + 4, kXS = kTN + 4;      // shared strides (4 mod 16 doubles: no bank conflicts)
 constexpr int kNT = 512;
+constexpr int kIA = kTK * kTM / kNT, kIB = kTK * kTN / kNT;   // elements of a slice per thread: 4 and 8
 constexpr i64 kMaxGridZ = 65535;
 constexpr size_t kSmem = sizeof(double) * kTK * (kLS + kXS);   // 51,200 bytes: dynamic shared memory
 
@@ -98,6 +99,38 @@ __global__ void embed_frame_kernel(int nBk, int nBall, const Ti *__restrict__ as
     rt[o] = neg ? -r[i] : r[i];
 }
 
+// A thread's elements of one K slice: items (row t / 64 + 8 it, column t % 64) of A and
+// (t / 128 + 4 it, t % 128) of B, zero where there is none.  Loaded for the next slice
+// while the current one is multiplied (the MMAs of a slice take ~4100 cycles; the loads,
+// two dependent lookups each, took twice that between them when they came first); the
+// signs wait until the elements are used, so that nothing waits for the loads before.
+// ADAPT screening at 20o 3+3 (tab_kernel 1.34 ms, pair2_kernel 0.36 of 4.14): 4.02 ->
+// 3.41 ms a step.
+struct Slice {
+    double a[kIA], b[kIB];
+    unsigned neg;
+    __device__ __forceinline__ void load_a(int it, const double *v, bool on, i64 i, int sign)
+    {
+        a[it] = on ? __ldg(v + i) : 0.0;
+        neg |= (unsigned)(sign & 1) << it;
+    }
+    __device__ __forceinline__ void load_b(int it, const double *v, bool on, i64 i, int sign)
+    {
+        b[it] = on ? __ldg(v + i) : 0.0;
+        neg |= (unsigned)(sign & 1) << (kIA + it);
+    }
+    __device__ __forceinline__ void put(double (*As)[kLS], double (*Bs)[kXS]) const
+    {
+        const int t = threadIdx.x;
+#pragma unroll
+        for (int it = 0; it < kIA; ++it)
+            As[t / kTM + it * (kNT / kTM)][t % kTM] = neg & (1u << it) ? -a[it] : a[it];
+#pragma unroll
+        for (int it = 0; it < kIB; ++it)
+            Bs[t / kTN + it * (kNT / kTN)][t % kTN] = neg & (1u << (kIA + it)) ? -b[it] : b[it];
+    }
+};
+
 // Accumulator of one 64 x 128 tile of C = A^T B: each step multiplies a 32-row K
 // slice held in shared memory (As[k][row], Bs[k][col]).  DMMA fragment mapping of
 // m8n8k4 row.col: lane (g, t) = (lane / 4, lane % 4) holds A[g][t], B[t][g] and
@@ -140,12 +173,6 @@ struct Acc {
     }
 };
 
-__device__ __forceinline__ double signed_at(const double *__restrict__ v, i64 i, int neg)
-{
-    const double x = __ldg(v + i);
-    return neg ? -x : x;
-}
-
 struct TabArgs {
     int n, nB, nHa, nHb, M, hsplit;
     const int *idxA;   // [nHa][n]
@@ -165,57 +192,46 @@ __global__ void __launch_bounds__(kNT, 1) tab_kernel(const TabArgs P)
     double(*Bs)[kXS] = reinterpret_cast<double(*)[kXS]>(smem_tab + kTK * kLS);
     const int m0 = blockIdx.x * kTM, c0 = blockIdx.y * kTN;
     const int hA0 = blockIdx.z * P.hsplit, hA1 = min(P.nHa, hA0 + P.hsplit);
-    constexpr int IA = kTK * kTM / kNT, IB = kTK * kTN / kNT;   // 4 and 8 fill items per thread
-    // fixed per thread: the item's slice row k and output index (p, r) or (q, s)
-    int ak[IA], ap[IA], ar[IA], bk[IB], bp[IB], br[IB];
+    // a thread's fill items share one output index, (p, r) of A and (q, s) of B, and
+    // are slice rows ak + 8 it and bk + 4 it
+    const int ja = (int)threadIdx.x % kTM, jb = (int)threadIdx.x % kTN;
+    const int ak = (int)threadIdx.x / kTM, bk = (int)threadIdx.x / kTN;
+    const bool va = m0 + ja < P.M, vb = c0 + jb < P.M;
+    const int ap = va ? (m0 + ja) / P.n : 0, ar = va ? (m0 + ja) % P.n : 0;
+    const int bp = vb ? (c0 + jb) / P.n : 0, br = vb ? (c0 + jb) % P.n : 0;
+    Slice X;   // the next slice, loaded while the current one is multiplied
+    auto load = [&](int hA, int hB0) {
+        const int ia = va ? __ldg(P.idxA + (i64)hA * P.n + ap) : -1;
+        const int ib = vb ? __ldg(P.idxA + (i64)hA * P.n + bp) : -1;
+        int qa[kIA], qb[kIB];
 #pragma unroll
-    for (int it = 0; it < IA; ++it) {
-        const int i = threadIdx.x + it * kNT, j = m0 + i % kTM;
-        ak[it] = i / kTM;
-        ap[it] = j < P.M ? j / P.n : -1;
-        ar[it] = j < P.M ? j % P.n : 0;
-    }
+        for (int it = 0; it < kIA; ++it) {
+            const int hB = hB0 + ak + it * (kNT / kTM);
+            qa[it] = ia >= 0 && hB < P.nHb ? __ldg(P.idxB + (i64)hB * P.n + ar) : -1;
+        }
 #pragma unroll
-    for (int it = 0; it < IB; ++it) {
-        const int i = threadIdx.x + it * kNT, j = c0 + i % kTN;
-        bk[it] = i / kTN;
-        bp[it] = j < P.M ? j / P.n : -1;
-        br[it] = j < P.M ? j % P.n : 0;
-    }
+        for (int it = 0; it < kIB; ++it) {
+            const int hB = hB0 + bk + it * (kNT / kTN);
+            qb[it] = ib >= 0 && hB < P.nHb ? __ldg(P.idxB + (i64)hB * P.n + br) : -1;
+        }
+        X.neg = 0;
+#pragma unroll
+        for (int it = 0; it < kIA; ++it) X.load_a(it, P.lt, qa[it] >= 0, (i64)(ia >> 1) * P.nB + (qa[it] >> 1), ia ^ qa[it]);
+#pragma unroll
+        for (int it = 0; it < kIB; ++it) X.load_b(it, P.rt, qb[it] >= 0, (i64)(ib >> 1) * P.nB + (qb[it] >> 1), ib ^ qb[it]);
+    };
     Acc acc;
     acc.zero();
-    for (int hA = hA0; hA < hA1; ++hA) {
-        int ia[IA], ib[IB];   // alpha side of every item is fixed for this hA
-#pragma unroll
-        for (int it = 0; it < IA; ++it) ia[it] = ap[it] >= 0 ? __ldg(P.idxA + (i64)hA * P.n + ap[it]) : -1;
-#pragma unroll
-        for (int it = 0; it < IB; ++it) ib[it] = bp[it] >= 0 ? __ldg(P.idxA + (i64)hA * P.n + bp[it]) : -1;
+    if (hA0 < hA1 && P.nHb > 0) load(hA0, 0);
+    for (int hA = hA0; hA < hA1; ++hA)
         for (int hB0 = 0; hB0 < P.nHb; hB0 += kTK) {
-#pragma unroll
-            for (int it = 0; it < IA; ++it) {
-                const int hB = hB0 + ak[it];
-                double v = 0.0;
-                if (ia[it] >= 0 && hB < P.nHb) {
-                    const int jb = __ldg(P.idxB + (i64)hB * P.n + ar[it]);
-                    if (jb >= 0) v = signed_at(P.lt, (i64)(ia[it] >> 1) * P.nB + (jb >> 1), (ia[it] ^ jb) & 1);
-                }
-                As[ak[it]][(threadIdx.x + it * kNT) % kTM] = v;
-            }
-#pragma unroll
-            for (int it = 0; it < IB; ++it) {
-                const int hB = hB0 + bk[it];
-                double v = 0.0;
-                if (ib[it] >= 0 && hB < P.nHb) {
-                    const int jb = __ldg(P.idxB + (i64)hB * P.n + br[it]);
-                    if (jb >= 0) v = signed_at(P.rt, (i64)(ib[it] >> 1) * P.nB + (jb >> 1), (ib[it] ^ jb) & 1);
-                }
-                Bs[bk[it]][(threadIdx.x + it * kNT) % kTN] = v;
-            }
+            X.put(As, Bs);
             __syncthreads();
+            if (hB0 + kTK < P.nHb) load(hA, hB0 + kTK);
+            else if (hA + 1 < hA1) load(hA + 1, 0);
             acc.step(As, Bs);
             __syncthreads();
         }
-    }
     acc.flush(P.C, P.M, m0, c0, P.M, P.M);
 }
 
@@ -241,51 +257,39 @@ __global__ void __launch_bounds__(kNT, 1) pair2_kernel(const PairArgs P)
     const int m0 = blockIdx.x * kTM, c0 = blockIdx.y * kTN;
     const int nos = (P.nO + P.osplit - 1) / P.osplit;
     const i64 nitems = (i64)P.nH2 * nos;
-    constexpr int IA = kTK * kTM / kNT, IB = kTK * kTN / kNT;
-    int ak[IA], ja[IA], bk[IB], jb[IB];   // per fill item: slice row and pair column (or -1)
+    const int ja = m0 + (int)threadIdx.x % kTM, jb = c0 + (int)threadIdx.x % kTN;   // pair columns
+    const int ak = (int)threadIdx.x / kTM, bk = (int)threadIdx.x / kTN;
+    Slice X;   // as in tab_kernel
+    auto load = [&](i64 item, int s0) {
+        const int h2 = (int)(item / nos), o1 = min(P.nO, (int)(item % nos) * P.osplit + P.osplit);
+        const int ia = ja < P.npair ? __ldg(P.idx2 + (i64)h2 * P.npair + ja) : -1;
+        const int ib = jb < P.npair ? __ldg(P.idx2 + (i64)h2 * P.npair + jb) : -1;
+        auto at = [&](int i, int o) {
+            return P.spin == 0 ? (i64)(i >> 1) * P.nB + o : (i64)o * P.nB + (i >> 1);
+        };
+        X.neg = 0;
 #pragma unroll
-    for (int it = 0; it < IA; ++it) {
-        const int i = threadIdx.x + it * kNT, j = m0 + i % kTM;
-        ak[it] = i / kTM;
-        ja[it] = j < P.npair ? j : -1;
-    }
+        for (int it = 0; it < kIA; ++it) {
+            const int o = s0 + ak + it * (kNT / kTM);
+            X.load_a(it, P.lt, ia >= 0 && o < o1, at(ia, o), ia);
+        }
 #pragma unroll
-    for (int it = 0; it < IB; ++it) {
-        const int i = threadIdx.x + it * kNT, j = c0 + i % kTN;
-        bk[it] = i / kTN;
-        jb[it] = j < P.npair ? j : -1;
-    }
+        for (int it = 0; it < kIB; ++it) {
+            const int o = s0 + bk + it * (kNT / kTN);
+            X.load_b(it, P.rt, ib >= 0 && o < o1, at(ib, o), ib);
+        }
+    };
     Acc acc;
     acc.zero();
+    if (blockIdx.z < nitems) load(blockIdx.z, (int)(blockIdx.z % nos) * P.osplit);
     for (i64 item = blockIdx.z; item < nitems; item += gridDim.z) {
-        const int h2 = (int)(item / nos), o0 = (int)(item % nos) * P.osplit, o1 = min(P.nO, o0 + P.osplit);
-        int ia[IA], ib[IB];
-#pragma unroll
-        for (int it = 0; it < IA; ++it) ia[it] = ja[it] >= 0 ? __ldg(P.idx2 + (i64)h2 * P.npair + ja[it]) : -1;
-#pragma unroll
-        for (int it = 0; it < IB; ++it) ib[it] = jb[it] >= 0 ? __ldg(P.idx2 + (i64)h2 * P.npair + jb[it]) : -1;
+        const int o0 = (int)(item % nos) * P.osplit, o1 = min(P.nO, o0 + P.osplit);
         for (int s0 = o0; s0 < o1; s0 += kTK) {
-#pragma unroll
-            for (int it = 0; it < IA; ++it) {
-                const int o = s0 + ak[it];
-                double v = 0.0;
-                if (ia[it] >= 0 && o < o1) {
-                    const i64 e = P.spin == 0 ? (i64)(ia[it] >> 1) * P.nB + o : (i64)o * P.nB + (ia[it] >> 1);
-                    v = signed_at(P.lt, e, ia[it] & 1);
-                }
-                As[ak[it]][(threadIdx.x + it * kNT) % kTM] = v;
-            }
-#pragma unroll
-            for (int it = 0; it < IB; ++it) {
-                const int o = s0 + bk[it];
-                double v = 0.0;
-                if (ib[it] >= 0 && o < o1) {
-                    const i64 e = P.spin == 0 ? (i64)(ib[it] >> 1) * P.nB + o : (i64)o * P.nB + (ib[it] >> 1);
-                    v = signed_at(P.rt, e, ib[it] & 1);
-                }
-                Bs[bk[it]][(threadIdx.x + it * kNT) % kTN] = v;
-            }
+            X.put(As, Bs);
             __syncthreads();
+            const i64 next = item + gridDim.z;
+            if (s0 + kTK < o1) load(item, s0 + kTK);
+            else if (next < nitems) load(next, (int)(next % nos) * P.osplit);
             acc.step(As, Bs);
             __syncthreads();
         }

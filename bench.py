@@ -330,10 +330,11 @@ def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma
             "dense_frac_of_measured_dmma_peak": (dense_total / max(1, n_launch) / per_launch_s / 1e12 / dmma_peak)
             if dense_total and dmma_peak else None,
             "note": "dominant kernel of the structured sigma, timed live per launch with CUDA events; achieved = "
-                    "its compulsory HBM bytes per launch / launch time, of the measured HBM copy peak; the kernel "
-                    "is bound by the tensor cores' FP64 (DMMA) pipe, see dense_frac_of_measured_dmma_peak (the dense "
-                    "GEMM as executed against the measured DMMA peak); traffic = ncu dram bytes of a 15-orbital "
-                    "launch scaled by determinants per launch"}
+                    "its compulsory HBM bytes per launch / launch time, of the measured HBM copy peak; the mixed GEMM "
+                    "runs as exact byte products on the integer tensor cores, bound by the L1 pipe of its gathers and "
+                    "stores; dense_frac_of_measured_dmma_peak sets the dense FP64 GEMM against the DMMA pipe that it "
+                    "does not use; traffic = ncu dram bytes of a 15-orbital launch of the DMMA kernel (the same rows "
+                    "read and Z written) scaled by determinants per launch"}
     return roof, launches
 
 

@@ -1294,7 +1294,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
         if (rows > 0) {   // split products; nothing reads c~ in floating point after this
             int *rexp = reinterpret_cast<int *>(ct + (size_t)P.nA * P.ldA);   // behind the rows (run_fast)
             double *Z = static_cast<double *>(z.p);
-            STAGE(tm, 3, s, rc = rows_to_fixed(ct, P.nA, P.ldA, rexp, s));
+            STAGE(tm, 0, s, rc = rows_to_fixed(ct, P.nA, P.ldA, rexp, s));
             if (rc != BSIM_OK) return rc;
             for (int z0 = c0; z0 < c1; z0 += (int)z.w) {
                 for (int jb = 0; jb < P.M; jb += rows) {

@@ -225,8 +225,7 @@ c64_list_hvec_kernel(const BasisView<Ti> B, int nBt, const int2 *__restrict__ ro
 
 // lists of one (basis, network), built with the first sigma
 struct C64Lists {
-    const void *basis = nullptr;
-    i64 dim = -1;
+    u64 basis = 0;           // serial of the basis they were made for
     bool ok = false;
     int nBt = 0, nrows = 0, ytiles = 0;
     Arena arena;
@@ -243,8 +242,7 @@ std::mutex g_c64_mu;
 template <typename Ti>
 int c64_build(const DevBasis<Ti> *B, const DevNet<Ti> *N, C64Lists *P, cudaStream_t s)
 {
-    P->basis = B;
-    P->dim = B->dim;
+    P->basis = B->serial;
     P->ok = false;
     if (N->ngs == 0 || N->ngs > 65535 || B->dim == 0) return BSIM_OK;
     std::vector<int2> row;
@@ -337,7 +335,7 @@ int c64_hvec(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, doub
     {
         std::lock_guard<std::mutex> lk(g_c64_mu);
         P = static_cast<C64Lists *>(N->c64_state);
-        if (P && (P->basis != B || P->dim != B->dim)) {
+        if (P && P->basis != B->serial) {
             delete P;
             P = nullptr;
             const_cast<DevNet<Ti> *>(N)->c64_state = nullptr;

@@ -69,6 +69,12 @@ static std::atomic<long long> g_device_allocs{0};
 void note_device_alloc() { g_device_allocs.fetch_add(1, std::memory_order_relaxed); }
 long long device_alloc_count() { return g_device_allocs.load(std::memory_order_relaxed); }
 
+u64 next_serial()
+{
+    static std::atomic<u64> n{0};
+    return n.fetch_add(1, std::memory_order_relaxed) + 1;
+}
+
 // ---- arena --------------------------------------------------------------------
 int Arena::reserve(size_t bytes)
 {

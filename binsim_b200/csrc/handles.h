@@ -60,9 +60,14 @@ struct Workspace {
     void release();
 };
 
+// A number that no other basis of the process has or had.  Plans that a network
+// keeps are found by it: a freed basis' address is soon another basis' address.
+u64 next_serial();
+
 template <typename Ti>
 struct DevBasis {
     unsigned magic = HandleMagic<Ti>::basis;
+    const u64 serial = next_serial();
     int norb = 0, num_irreps = 0, num_blocks = 0;
     int nel_a = 0, nel_b = 0;
     i64 dim = 0, total_sym = 0;

@@ -41,8 +41,7 @@ constexpr int kBatchRows = 16;   // alpha entries per tile of the batched gradie
 
 template <typename Ti>
 struct PairPlan {
-    const void *basis = nullptr;
-    i64 basis_dim = -1;
+    u64 basis = 0;             // serial of the basis it was made for
     bool ok = false;
     std::vector<int4> desc;        // per group: {alpha offset or -1, alpha count, beta offset or -1, beta count}
     Arena arena;
@@ -66,8 +65,7 @@ std::mutex g_pair_mu;
 template <typename Ti>
 int build_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> *P)
 {
-    P->basis = B;
-    P->basis_dim = B->dim;
+    P->basis = B->serial;
     P->ok = false;
     if (B->num_blocks != 1) return BSIM_OK;
     const int nA = B->na[0], nB = B->nb[0];
@@ -141,7 +139,7 @@ int get_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> **out
 {
     std::lock_guard<std::mutex> lk(g_pair_mu);
     auto *p = static_cast<PairPlan<Ti> *>(N->pair_state);
-    if (p && p->basis == B && p->basis_dim == B->dim) { *out = p; return BSIM_OK; }
+    if (p && p->basis == B->serial) { *out = p; return BSIM_OK; }
     if (p) { delete p; const_cast<DevNet<Ti> *>(N)->pair_state = nullptr; }
     p = new PairPlan<Ti>();
     int rc = build_pair_plan(B, N, p);
@@ -158,7 +156,7 @@ PairPlan<Ti> *find_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N)
 {
     std::lock_guard<std::mutex> lk(g_pair_mu);
     auto *p = static_cast<PairPlan<Ti> *>(N->pair_state);
-    return (p && p->basis == B && p->basis_dim == B->dim) ? p : nullptr;
+    return (p && p->basis == B->serial) ? p : nullptr;
 }
 
 struct ListArgs {

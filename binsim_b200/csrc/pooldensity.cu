@@ -618,8 +618,7 @@ __global__ void theta_zero_kernel(const double *__restrict__ thetas, i64 n, int 
 }  // namespace
 
 struct DensityRoute {
-    const void *basis = nullptr;
-    i64 basis_dim = 0;
+    u64 basis = 0;                   // serial of the basis it was made for
     bool ok = false;                 // false: the route does not apply to this (basis, network)
     i64 ngs = 0;
     PoolDensity *P = nullptr;
@@ -647,14 +646,13 @@ int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute **out
     if (off || N->cplx || B->nel_a < 1 || B->nel_b < 1 || B->dim == 0 || N->ngs == 0 || B->norb > 64) return BSIM_OK;
     std::lock_guard<std::mutex> lk(g_route_mu);
     auto *R = static_cast<DensityRoute *>(N->density_state);
-    if (R && R->basis == B && R->basis_dim == B->dim) {
+    if (R && R->basis == B->serial) {
         *out = R->ok ? R : nullptr;
         return BSIM_OK;
     }
     if (R) { delete R; const_cast<DevNet<Ti> *>(N)->density_state = nullptr; }
     R = new DensityRoute;
-    R->basis = B;
-    R->basis_dim = B->dim;
+    R->basis = B->serial;
     R->ngs = N->ngs;
     auto &net = const_cast<DevNet<Ti> &>(*N);
     net.density_state = R;

@@ -171,8 +171,7 @@ blk_sigma_kernel(const BlkView V, const Ti *__restrict__ bstr, const double *__r
 
 template <typename Ti>
 struct BlkPlan {
-    const void *basis = nullptr;
-    i64 basis_dim = -1;
+    u64 basis = 0;                        // serial of the basis it was made for
     bool ok = false;
     Arena arena;
     BlkView v{};
@@ -210,8 +209,7 @@ u64 mask_above_odd(u64 x, int norb)   // orbitals with an odd number of x bits a
 template <typename Ti>
 int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
 {
-    P->basis = B;
-    P->basis_dim = B->dim;
+    P->basis = B->serial;
     P->ok = false;
     const int norb = B->norb, nirr = B->num_irreps;
     if (B->num_blocks < 2 || norb > 63 || N->norb > norb || N->cplx) return BSIM_OK;
@@ -528,7 +526,7 @@ int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, 
     {
         std::lock_guard<std::mutex> lk(g_blk_mu);
         P = static_cast<BlkPlan<Ti> *>(N->blk_state);
-        if (P && (P->basis != B || P->basis_dim != B->dim)) {
+        if (P && P->basis != B->serial) {
             delete P;
             P = nullptr;
             const_cast<DevNet<Ti> *>(N)->blk_state = nullptr;

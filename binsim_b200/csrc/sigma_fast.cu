@@ -1085,7 +1085,7 @@ static int get_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> **
 {
     std::lock_guard<std::mutex> lk(g_fast_mu);
     auto *st = static_cast<FastState<Ti> *>(N->fast_state);
-    if (st && st->plan.basis == B && st->plan.basis_dim == B->dim) { *out = st; return BSIM_OK; }
+    if (st && st->plan.basis == B->serial) { *out = st; return BSIM_OK; }
     if (st) { delete st; const_cast<DevNet<Ti> *>(N)->fast_state = nullptr; }
     st = new FastState<Ti>();
     int rc = build_fast_plan(B, N, &st->plan);

@@ -76,17 +76,17 @@ int batchgrad(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *thetas, 
     // ADAPT screening (every theta zero): the groups of the planned forms go
     // through the transition densities; whether every theta is zero is decided
     // on the device, so the call stays asynchronous
-    DensityRoute *D = nullptr;
+    std::shared_ptr<DensityRoute> D;
     int st = B->dim > 0 ? density_route(B, N, &D) : BSIM_OK;
     if (st != BSIM_OK) return st;
     const unsigned char *skip = nullptr;
     const int *flag = nullptr;
     if (D) {
-        if ((st = density_route_begin(D, thetas, s)) != BSIM_OK) return st;
-        skip = density_route_skip(D);
-        flag = density_route_flag(D);
+        if ((st = density_route_begin(D.get(), thetas, s)) != BSIM_OK) return st;
+        skip = density_route_skip(D.get());
+        flag = density_route_flag(D.get());
     }
-    auto finish = [&]() { return D ? density_route_finish<Ti>(D, l, r, grads, s) : BSIM_OK; };
+    auto finish = [&]() { return D ? density_route_finish<Ti>(D.get(), l, r, grads, s) : BSIM_OK; };
     if (B->dim > 0) {   // single-block bases: one launch over the groups' pair lists
         bool used = false;
         int st0 = pair_list_batchgrad(B, N, thetas, l, r, grads, s, &used, skip, flag);

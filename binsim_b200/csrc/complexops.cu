@@ -20,7 +20,7 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
+#include <memory>
 #include <unordered_map>
 #include <vector>
 
@@ -225,7 +225,6 @@ c64_list_hvec_kernel(const BasisView<Ti> B, int nBt, const int2 *__restrict__ ro
 
 // lists of one (basis, network), built with the first sigma
 struct C64Lists {
-    u64 basis = 0;           // serial of the basis they were made for
     bool ok = false;
     int nBt = 0, nrows = 0, ytiles = 0;
     Arena arena;
@@ -237,12 +236,9 @@ struct C64Lists {
     ~C64Lists() { arena.release(); }
 };
 
-std::mutex g_c64_mu;
-
 template <typename Ti>
 int c64_build(const DevBasis<Ti> *B, const DevNet<Ti> *N, C64Lists *P, cudaStream_t s)
 {
-    P->basis = B->serial;
     P->ok = false;
     if (N->ngs == 0 || N->ngs > 65535 || B->dim == 0) return BSIM_OK;
     std::vector<int2> row;
@@ -331,24 +327,18 @@ template <typename Ti>
 int c64_hvec(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, double *dst, cudaStream_t s)
 {
     if (B->dim == 0) return BSIM_OK;
-    C64Lists *P = nullptr;
-    {
-        std::lock_guard<std::mutex> lk(g_c64_mu);
-        P = static_cast<C64Lists *>(N->c64_state);
-        if (P && P->basis != B->serial) {
-            delete P;
-            P = nullptr;
-            const_cast<DevNet<Ti> *>(N)->c64_state = nullptr;
-        }
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (!P) BSIM_CUDA(cudaStreamIsCapturing(s, &cap));
-        if (!P && cap == cudaStreamCaptureStatusNone) {   // building allocates and waits: not inside a capture
-            P = new C64Lists();
-            const int st = c64_build(B, N, P, s);
-            if (st != BSIM_OK && st != BSIM_ERR_ALLOC) { delete P; return st; }
-            const_cast<DevNet<Ti> *>(N)->c64_state = P;
-            const_cast<DevNet<Ti> *>(N)->c64_free = [](void *q) { delete static_cast<C64Lists *>(q); };
-        }
+    std::shared_ptr<C64Lists> P = N->c64_plans.template find<C64Lists>(B->serial);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!P) BSIM_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (!P && cap == cudaStreamCaptureStatusNone) {   // building allocates and waits: not inside a capture
+        const int st = N->c64_plans.get(B->serial, &P, [&](std::shared_ptr<C64Lists> &plan) -> int {
+            auto p = std::make_shared<C64Lists>();
+            const int rc = c64_build(B, N, p.get(), s);
+            if (rc != BSIM_OK && rc != BSIM_ERR_ALLOC) return rc;
+            plan = p;
+            return BSIM_OK;
+        });
+        if (st != BSIM_OK) return st;
     }
     const cx *x = reinterpret_cast<const cx *>(src);
     cx *y = reinterpret_cast<cx *>(dst);

@@ -93,7 +93,6 @@ template <typename Ti>
 int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
 {
     P->ok = false;
-    P->basis = B->serial;
     if (B->num_blocks != 1) { P->why = "more than one symmetry block"; return BSIM_OK; }
     const int norb = B->norb;
     const int nA = B->na[0], nB = B->nb[0];

@@ -78,7 +78,6 @@ template <typename Ti>
 struct FastPlan {
     bool ok = false;
     std::string why;           // reason when the fast path is off
-    u64 basis = 0;             // serial of the basis it was made for
     int norb = 0, nA = 0, nB = 0, nelA = 0, nelB = 0;
     // padded row strides: ldA for rows of c~ (alpha rows, beta columns; at least one
     // padding column, a zero that the gather tables can name), ldB for

@@ -75,6 +75,47 @@ u64 next_serial()
     return n.fetch_add(1, std::memory_order_relaxed) + 1;
 }
 
+// ---- plans ----------------------------------------------------------------------
+namespace {
+struct PlanCaches {   // every live cache; never destroyed, handles may outlive static objects
+    std::mutex mu;
+    std::vector<PlanCache *> all;
+};
+PlanCaches &plan_caches()
+{
+    static PlanCaches *c = new PlanCaches;
+    return *c;
+}
+}  // namespace
+
+PlanCache::PlanCache(size_t keep) : keep_(keep)
+{
+    PlanCaches &c = plan_caches();
+    std::lock_guard<std::mutex> lk(c.mu);
+    c.all.push_back(this);
+}
+
+PlanCache::~PlanCache()
+{
+    PlanCaches &c = plan_caches();
+    std::lock_guard<std::mutex> lk(c.mu);
+    c.all.erase(std::find(c.all.begin(), c.all.end(), this));
+}
+
+void PlanCache::forget(u64 basis)
+{
+    std::lock_guard<std::mutex> lk(mu_);
+    slots_.erase(std::remove_if(slots_.begin(), slots_.end(), [&](const Slot &s) { return s.basis == basis; }),
+                 slots_.end());
+}
+
+void forget_basis(u64 basis)
+{
+    PlanCaches &c = plan_caches();
+    std::lock_guard<std::mutex> lk(c.mu);
+    for (PlanCache *p : c.all) p->forget(basis);
+}
+
 // ---- arena --------------------------------------------------------------------
 int Arena::reserve(size_t bytes)
 {

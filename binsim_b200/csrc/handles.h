@@ -6,6 +6,10 @@
 #pragma once
 #include "common.cuh"
 
+#include <memory>
+#include <mutex>
+#include <vector>
+
 namespace bsim {
 
 // Magic words per string type: UInt32 handles (the reference's GPU library's
@@ -64,6 +68,54 @@ struct Workspace {
 // keeps are found by it: a freed basis' address is soon another basis' address.
 u64 next_serial();
 
+// The plans of one kind that a network keeps, one per basis it is used with.  A
+// caller holds its plan by a shared pointer, so another thread that uses the network
+// with another basis cannot free it under the caller.  Plans go with their basis or
+// their network.
+class PlanCache {
+public:
+    explicit PlanCache(size_t keep);   // at most so many bases; the oldest plan goes first
+    ~PlanCache();
+    PlanCache(const PlanCache &) = delete;
+    PlanCache &operator=(const PlanCache &) = delete;
+    // The basis' plan; make(std::shared_ptr<T> &) makes a missing one, with room for it
+    // already made.  What make leaves in its argument is kept, whatever it returns.
+    template <typename T, typename Make>
+    int get(u64 basis, std::shared_ptr<T> *out, Make &&make)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        std::shared_ptr<T> p = std::static_pointer_cast<T>(lookup(basis));
+        int st = 0;
+        if (!p) {
+            while (slots_.size() >= keep_) slots_.erase(slots_.begin());
+            st = make(p);
+            if (p) slots_.push_back(Slot{basis, p});
+        }
+        *out = std::move(p);
+        return st;
+    }
+    template <typename T>
+    std::shared_ptr<T> find(u64 basis)   // null when there is none
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        return std::static_pointer_cast<T>(lookup(basis));
+    }
+    void forget(u64 basis);
+private:
+    struct Slot { u64 basis; std::shared_ptr<void> plan; };
+    std::shared_ptr<void> lookup(u64 basis) const
+    {
+        for (const Slot &s : slots_)
+            if (s.basis == basis) return s.plan;
+        return nullptr;
+    }
+    std::mutex mu_;
+    const size_t keep_;
+    std::vector<Slot> slots_;
+};
+constexpr size_t kEveryBasis = ~size_t(0);
+void forget_basis(u64 basis);   // drops its plans from every network
+
 template <typename Ti>
 struct DevBasis {
     unsigned magic = HandleMagic<Ti>::basis;
@@ -84,7 +136,7 @@ struct DevBasis {
 
     int upload();                       // builds dense maps + copies tables
     i64 find_det(u64 astr, u64 bstr) const;   // -1 when absent
-    ~DevBasis() { ws.release(); arena.release(); magic = 0; }
+    ~DevBasis() { forget_basis(serial); ws.release(); arena.release(); magic = 0; }
 };
 
 template <typename Ti>
@@ -113,35 +165,20 @@ struct DevNet {
     const int *d_plan_groups = nullptr;
     const int4 *d_plan_chunks = nullptr;
 
-    // cached structured-sigma plan for the last basis it was used with
-    void *fast_state = nullptr;
-    void (*fast_free)(void *) = nullptr;
-    // cached pair lists of the pair operators for the last basis they were used with
-    void *pair_state = nullptr;
-    void (*pair_free)(void *) = nullptr;
-    // cached theta = 0 route of the pool gradient (transition densities) for the
-    // last basis it was used with
-    void *density_state = nullptr;
-    void (*density_free)(void *) = nullptr;
-
-    // cached row lists of the complex sigma
-    void *c64_state = nullptr;
-    void (*c64_free)(void *) = nullptr;
-    // cached sigma plan of a symmetry-blocked basis
-    void *blk_state = nullptr;
-    void (*blk_free)(void *) = nullptr;
+    // structured-sigma plan, pair lists of the pair operators and theta = 0 route of
+    // the pool gradient (transition densities) for the last basis each was used with;
+    // large, with scratch
+    mutable PlanCache fast_plans{1}, pair_plans{1}, density_plans{1};
+    // sigma plans of symmetry-blocked bases, row lists of the complex sigma: of every
+    // basis, so that bases in turn (the irreps of a molecule) do not make them again
+    mutable PlanCache blk_plans{kEveryBasis}, c64_plans{kEveryBasis};
     // cached forms of the groups as excitations (rotation sequences)
     void *rot_state = nullptr;
     void (*rot_free)(void *) = nullptr;
 
     int finalize();   // derived tables + upload
     ~DevNet() {
-        if (fast_state && fast_free) fast_free(fast_state);
-        if (pair_state && pair_free) pair_free(pair_state);
-        if (density_state && density_free) density_free(density_state);
         if (rot_state && rot_free) rot_free(rot_state);
-        if (blk_state && blk_free) blk_free(blk_state);
-        if (c64_state && c64_free) c64_free(c64_state);
         arena.release();
         magic = 0;
     }

@@ -124,7 +124,7 @@ int pair_list_batchgrad(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double
 // the flag is set, overwrite grads of the planned groups.
 struct DensityRoute;
 template <typename Ti>
-int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute **out);
+int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::shared_ptr<DensityRoute> *out);
 int density_route_begin(DensityRoute *D, const double *thetas, cudaStream_t s);
 template <typename Ti>
 int density_route_finish(DensityRoute *D, const double *l, const double *r, double *grads, cudaStream_t s);

@@ -41,7 +41,6 @@ constexpr int kBatchRows = 16;   // alpha entries per tile of the batched gradie
 
 template <typename Ti>
 struct PairPlan {
-    u64 basis = 0;             // serial of the basis it was made for
     bool ok = false;
     std::vector<int4> desc;        // per group: {alpha offset or -1, alpha count, beta offset or -1, beta count}
     Arena arena;
@@ -60,12 +59,9 @@ struct PairPlan {
     }
 };
 
-std::mutex g_pair_mu;
-
 template <typename Ti>
 int build_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> *P)
 {
-    P->basis = B->serial;
     P->ok = false;
     if (B->num_blocks != 1) return BSIM_OK;
     const int nA = B->na[0], nB = B->nb[0];
@@ -135,28 +131,21 @@ int build_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> *P)
 }
 
 template <typename Ti>
-int get_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> **out)
+int get_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::shared_ptr<PairPlan<Ti>> *out)
 {
-    std::lock_guard<std::mutex> lk(g_pair_mu);
-    auto *p = static_cast<PairPlan<Ti> *>(N->pair_state);
-    if (p && p->basis == B->serial) { *out = p; return BSIM_OK; }
-    if (p) { delete p; const_cast<DevNet<Ti> *>(N)->pair_state = nullptr; }
-    p = new PairPlan<Ti>();
-    int rc = build_pair_plan(B, N, p);
-    if (rc != BSIM_OK) { delete p; return rc; }
-    const_cast<DevNet<Ti> *>(N)->pair_state = p;
-    const_cast<DevNet<Ti> *>(N)->pair_free = [](void *q) { delete static_cast<PairPlan<Ti> *>(q); };
-    *out = p;
-    return BSIM_OK;
+    return N->pair_plans.get(B->serial, out, [&](std::shared_ptr<PairPlan<Ti>> &p) {
+        auto plan = std::make_shared<PairPlan<Ti>>();
+        const int rc = build_pair_plan(B, N, plan.get());
+        if (rc == BSIM_OK) p = plan;
+        return rc;
+    });
 }
 
 // The cached plan of (B, N) if one exists; never builds one (no allocation).
 template <typename Ti>
-PairPlan<Ti> *find_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N)
+std::shared_ptr<PairPlan<Ti>> find_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N)
 {
-    std::lock_guard<std::mutex> lk(g_pair_mu);
-    auto *p = static_cast<PairPlan<Ti> *>(N->pair_state);
-    return (p && p->basis == B->serial) ? p : nullptr;
+    return N->pair_plans.template find<PairPlan<Ti>>(B->serial);
 }
 
 struct ListArgs {
@@ -470,7 +459,7 @@ int pair_list_launch(const DevBasis<Ti> *B, const DevNet<Ti> *N, i64 gidx, PairA
                      cudaStream_t s, bool *used, bool may_build)
 {
     *used = false;
-    PairPlan<Ti> *P = nullptr;
+    std::shared_ptr<PairPlan<Ti>> P;
     if (may_build) {
         int st = get_pair_plan(B, N, &P);
         if (st != BSIM_OK) return st;
@@ -506,7 +495,7 @@ int pair_list_batchgrad(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double
                         const int *flag)
 {
     *used = false;
-    PairPlan<Ti> *P = nullptr;
+    std::shared_ptr<PairPlan<Ti>> P;
     int st = get_pair_plan(B, N, &P);
     if (st != BSIM_OK) return st;
     if (!P->ok) return BSIM_OK;

@@ -618,7 +618,6 @@ __global__ void theta_zero_kernel(const double *__restrict__ thetas, i64 n, int 
 }  // namespace
 
 struct DensityRoute {
-    u64 basis = 0;                   // serial of the basis it was made for
     bool ok = false;                 // false: the route does not apply to this (basis, network)
     i64 ngs = 0;
     PoolDensity *P = nullptr;
@@ -628,35 +627,36 @@ struct DensityRoute {
     ~DensityRoute() { delete P; arena.release(); }
 };
 
-static std::mutex g_route_mu;
-
 // Route for (B, N): groups classified by bsim_poolplan_classify from the
 // network's host copy; applies when some group has a planned form and the
 // dense tables take at most half of the free device memory (a blocked basis
 // only when its union string arrays hold at most 4x its determinants).
 // BSIM_POOL_DENSITY=0 turns the route off.
 template <typename Ti>
-int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute **out)
+static int make_density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute *R);
+
+template <typename Ti>
+int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::shared_ptr<DensityRoute> *out)
 {
-    *out = nullptr;
+    out->reset();
     static const bool off = [] {
         const char *e = getenv("BSIM_POOL_DENSITY");
         return e && e[0] == '0';
     }();
     if (off || N->cplx || B->nel_a < 1 || B->nel_b < 1 || B->dim == 0 || N->ngs == 0 || B->norb > 64) return BSIM_OK;
-    std::lock_guard<std::mutex> lk(g_route_mu);
-    auto *R = static_cast<DensityRoute *>(N->density_state);
-    if (R && R->basis == B->serial) {
-        *out = R->ok ? R : nullptr;
-        return BSIM_OK;
-    }
-    if (R) { delete R; const_cast<DevNet<Ti> *>(N)->density_state = nullptr; }
-    R = new DensityRoute;
-    R->basis = B->serial;
+    std::shared_ptr<DensityRoute> R;
+    const int st = N->density_plans.get(B->serial, &R, [&](std::shared_ptr<DensityRoute> &p) {
+        p = std::make_shared<DensityRoute>();
+        return make_density_route(B, N, p.get());
+    });
+    if (st == BSIM_OK && R->ok) *out = R;
+    return st;
+}
+
+template <typename Ti>
+static int make_density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute *R)
+{
     R->ngs = N->ngs;
-    auto &net = const_cast<DevNet<Ti> &>(*N);
-    net.density_state = R;
-    net.density_free = [](void *q) { delete static_cast<DensityRoute *>(q); };
     // the network in the flat form of bsim_poolplan_classify
     const i64 ngs = N->ngs;
     std::vector<uint64_t> axs(ngs), bxs(ngs), za, zb;
@@ -704,7 +704,6 @@ int density_route(const DevBasis<Ti> *B, const DevNet<Ti> *N, DensityRoute **out
     R->skip = R->arena.take<unsigned char>(ngs);
     BSIM_CUDA(cudaMemcpy(R->skip, skip.data(), (size_t)ngs, cudaMemcpyHostToDevice));
     R->ok = true;
-    *out = R;
     return BSIM_OK;
 }
 
@@ -726,9 +725,11 @@ int density_route_finish(DensityRoute *D, const double *l, const double *r, doub
 const unsigned char *density_route_skip(const DensityRoute *D) { return D->skip; }
 const int *density_route_flag(const DensityRoute *D) { return D->flag; }
 
-template int density_route<unsigned>(const DevBasis<unsigned> *, const DevNet<unsigned> *, DensityRoute **);
+template int density_route<unsigned>(const DevBasis<unsigned> *, const DevNet<unsigned> *,
+                                     std::shared_ptr<DensityRoute> *);
 template int density_route<unsigned long long>(const DevBasis<unsigned long long> *,
-                                               const DevNet<unsigned long long> *, DensityRoute **);
+                                               const DevNet<unsigned long long> *,
+                                               std::shared_ptr<DensityRoute> *);
 template int density_route_finish<unsigned>(DensityRoute *, const double *, const double *, double *, cudaStream_t);
 template int density_route_finish<unsigned long long>(DensityRoute *, const double *, const double *, double *,
                                                       cudaStream_t);

@@ -25,7 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
+#include <memory>
 #include <unordered_map>
 
 namespace bsim {
@@ -171,7 +171,6 @@ blk_sigma_kernel(const BlkView V, const Ti *__restrict__ bstr, const double *__r
 
 template <typename Ti>
 struct BlkPlan {
-    u64 basis = 0;                        // serial of the basis it was made for
     bool ok = false;
     Arena arena;
     BlkView v{};
@@ -186,8 +185,6 @@ struct BlkPlan {
         if (ct) cudaFree(ct);
     }
 };
-
-std::mutex g_blk_mu;
 
 inline int popc(u64 x) { return __builtin_popcountll(x); }
 
@@ -209,7 +206,6 @@ u64 mask_above_odd(u64 x, int norb)   // orbitals with an odd number of x bits a
 template <typename Ti>
 int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
 {
-    P->basis = B->serial;
     P->ok = false;
     const int norb = B->norb, nirr = B->num_irreps;
     if (B->num_blocks < 2 || norb > 63 || N->norb > norb || N->cplx) return BSIM_OK;
@@ -522,35 +518,26 @@ int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, 
 {
     *used = false;
     if (B->num_blocks < 2) return BSIM_OK;
-    BlkPlan<Ti> *P = nullptr;
-    {
-        std::lock_guard<std::mutex> lk(g_blk_mu);
-        P = static_cast<BlkPlan<Ti> *>(N->blk_state);
-        if (P && P->basis != B->serial) {
-            delete P;
-            P = nullptr;
-            const_cast<DevNet<Ti> *>(N)->blk_state = nullptr;
-        }
-        if (!P) {
-            P = new BlkPlan<Ti>();
-            int rc = build(B, N, P);
-            if (rc == BSIM_OK && P->ok) {
-                const cudaError_t e = dmalloc(&P->ct, sizeof(double) * B->dim);
-                if (e != cudaSuccess) {
-                    P->ct = nullptr;
-                    rc = e == cudaErrorMemoryAllocation ? BSIM_ERR_ALLOC : cuda_status(e, "symmetry-blocked sigma");
-                }
+    std::shared_ptr<BlkPlan<Ti>> P;
+    const int st = N->blk_plans.get(B->serial, &P, [&](std::shared_ptr<BlkPlan<Ti>> &plan) {
+        auto p = std::make_shared<BlkPlan<Ti>>();
+        int rc = build(B, N, p.get());
+        if (rc == BSIM_OK && p->ok) {
+            const cudaError_t e = dmalloc(&p->ct, sizeof(double) * B->dim);
+            if (e != cudaSuccess) {
+                p->ct = nullptr;
+                rc = e == cudaErrorMemoryAllocation ? BSIM_ERR_ALLOC : cuda_status(e, "symmetry-blocked sigma");
             }
-            if (rc == BSIM_ERR_ALLOC) {   // no room for the lists: the tile kernel needs none
-                (void)cudaGetLastError();
-                P->ok = false;
-                rc = BSIM_OK;
-            }
-            if (rc != BSIM_OK) { delete P; return rc; }
-            const_cast<DevNet<Ti> *>(N)->blk_state = P;
-            const_cast<DevNet<Ti> *>(N)->blk_free = [](void *q) { delete static_cast<BlkPlan<Ti> *>(q); };
         }
-    }
+        if (rc == BSIM_ERR_ALLOC) {   // no room for the lists: the tile kernel needs none
+            (void)cudaGetLastError();
+            p->ok = false;
+            rc = BSIM_OK;
+        }
+        if (rc == BSIM_OK) plan = p;
+        return rc;
+    });
+    if (st != BSIM_OK) return st;
     if (!P->ok) return BSIM_OK;
     if (src32) blk_frame_kernel<Ti, float><<<P->v.nAt, 256, 0, s>>>(P->v, B->view.bstrs, src32, P->ct);
     else blk_frame_kernel<Ti, double><<<P->v.nAt, 256, 0, s>>>(P->v, B->view.bstrs, src, P->ct);

@@ -25,7 +25,7 @@
 
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
+#include <memory>
 #include <type_traits>
 
 namespace bsim {
@@ -1078,22 +1078,15 @@ struct FastState {
     FastScratch<Ti> scratch;
 };
 
-static std::mutex g_fast_mu;
-
 template <typename Ti>
-static int get_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> **out)
+static int get_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::shared_ptr<FastState<Ti>> *out)
 {
-    std::lock_guard<std::mutex> lk(g_fast_mu);
-    auto *st = static_cast<FastState<Ti> *>(N->fast_state);
-    if (st && st->plan.basis == B->serial) { *out = st; return BSIM_OK; }
-    if (st) { delete st; const_cast<DevNet<Ti> *>(N)->fast_state = nullptr; }
-    st = new FastState<Ti>();
-    int rc = build_fast_plan(B, N, &st->plan);
-    if (rc != BSIM_OK) { delete st; return rc; }
-    const_cast<DevNet<Ti> *>(N)->fast_state = st;
-    const_cast<DevNet<Ti> *>(N)->fast_free = [](void *p) { delete static_cast<FastState<Ti> *>(p); };
-    *out = st;
-    return BSIM_OK;
+    return N->fast_plans.get(B->serial, out, [&](std::shared_ptr<FastState<Ti>> &p) {
+        auto st = std::make_shared<FastState<Ti>>();
+        const int rc = build_fast_plan(B, N, &st->plan);
+        if (rc == BSIM_OK) p = st;
+        return rc;
+    });
 }
 
 static size_t scratch_limit()
@@ -1156,7 +1149,7 @@ static int z_slot(void **zbuf, size_t *zhave, void *spare, size_t spare_n, size_
 template <typename Ti>
 bool fast_sigma_available(const DevBasis<Ti> *B, const DevNet<Ti> *N)
 {
-    FastState<Ti> *st = nullptr;
+    std::shared_ptr<FastState<Ti>> st;
     if (get_fast(B, N, &st) != BSIM_OK) return false;
     return st->plan.ok;
 }
@@ -1508,12 +1501,12 @@ static int sigma_fast_impl(const DevBasis<Ti> *B, const DevNet<Ti> *N, const dou
                            double *dst, bool mixed, cudaStream_t s, bool *used, StageTimer *tm)
 {
     *used = false;
-    FastState<Ti> *st = nullptr;
+    std::shared_ptr<FastState<Ti>> st;
     int rc = get_fast(B, N, &st);
     if (rc != BSIM_OK) return rc;
     if (!st->plan.ok) return BSIM_OK;
-    rc = mixed ? run_fast<Ti, float>(B, N, st, src, src32, dst, 0, st->plan.nB, s, tm)
-               : run_fast<Ti, double>(B, N, st, src, nullptr, dst, 0, st->plan.nB, s, tm);
+    rc = mixed ? run_fast<Ti, float>(B, N, st.get(), src, src32, dst, 0, st->plan.nB, s, tm)
+               : run_fast<Ti, double>(B, N, st.get(), src, nullptr, dst, 0, st->plan.nB, s, tm);
     if (rc != BSIM_OK) return rc;
     if (!st->plan.residual.empty()) {
         STAGE(tm, 6, s, rc = sigma_generic_accumulate(B, N, st->plan.d_resid, st->plan.d_resid_chunks,
@@ -1535,7 +1528,7 @@ template <typename Ti>
 int sigma_fast_cols(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, double *dst, bool mixed,
                     i64 col_lo, i64 col_hi, cudaStream_t s)
 {
-    FastState<Ti> *st = nullptr;
+    std::shared_ptr<FastState<Ti>> st;
     int rc = get_fast(B, N, &st);
     if (rc != BSIM_OK) return rc;
     const FastPlan<Ti> &P = st->plan;
@@ -1550,8 +1543,8 @@ int sigma_fast_cols(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *sr
         return BSIM_ERR_ARG;
     }
     if (col_lo == col_hi) return BSIM_OK;
-    return mixed ? run_fast<Ti, float>(B, N, st, src, nullptr, dst, (int)col_lo, (int)col_hi, s, nullptr)
-                 : run_fast<Ti, double>(B, N, st, src, nullptr, dst, (int)col_lo, (int)col_hi, s, nullptr);
+    return mixed ? run_fast<Ti, float>(B, N, st.get(), src, nullptr, dst, (int)col_lo, (int)col_hi, s, nullptr)
+                 : run_fast<Ti, double>(B, N, st.get(), src, nullptr, dst, (int)col_lo, (int)col_hi, s, nullptr);
 }
 
 template <typename Ti>
@@ -1569,7 +1562,7 @@ int sigma_fast_stages(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *
 template <typename Ti>
 int fast_sigma_info(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::string *why, int *nresid)
 {
-    FastState<Ti> *st = nullptr;
+    std::shared_ptr<FastState<Ti>> st;
     int rc = get_fast(B, N, &st);
     if (rc != BSIM_OK) return rc;
     *why = st->plan.ok ? std::string("structured") + (st->plan.riA.on ? " ri-alpha" : "") +

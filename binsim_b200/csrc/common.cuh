@@ -73,6 +73,20 @@ inline cudaError_t dmalloc_async(T **p, size_t bytes, cudaStream_t s)
         if (e__ != cudaSuccess) return ::bsim::cuda_status(e__, #call); \
     } while (0)
 
+// Shared memory of a CTA, static and dynamic.
+constexpr size_t kSmemMax = 227 * 1024;
+// Lets a kernel be launched with any dynamic shared memory that fits.  The limit
+// belongs to the kernel and not to a launch, so it is the same value in every call: one
+// that followed the launch's size would fail another thread's larger launch.
+template <typename... KArgs>
+inline cudaError_t allow_smem(void (*kern)(KArgs...))
+{
+    cudaFuncAttributes a{};
+    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemMax - a.sharedSizeBytes));
+}
+
 // Chained launches (programmatic dependent launch): the kernel's CTAs may become
 // resident while the stream's previous kernel finishes; chain_wait(), before the
 // kernel touches anything an earlier one wrote, waits until that kernel has

@@ -582,8 +582,7 @@ int dav_eigh_dev(int k, const double *h, int ldh, double *evals, double *evecs, 
 {
     if (k < 1 || k > kMaxSub) { set_error("subspace size %d out of range", k); return BSIM_ERR_ARG; }
     const int smem = (int)(sizeof(double) * 2 * k * k);   // <= 64 KB (k <= 64)
-    if (smem > 48 * 1024)
-        BSIM_CUDA(cudaFuncSetAttribute(eigh_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (smem > 48 * 1024) BSIM_CUDA(allow_smem(eigh_kernel));
     eigh_kernel<<<1, 32, smem, s>>>(k, h, ldh, evals, evecs);
     BSIM_CUDA(cudaGetLastError());
     return BSIM_OK;

@@ -141,7 +141,6 @@ inline size_t ri_smem_bytes(int nU, size_t elem)
 // global memory), Lam_conn [K x 64] (or one 32-row F chunk of it), an X slice
 // [32 x kMixCols] and the connected-excitation lists.
 constexpr int kMaxConn = 128;   // connected alpha singles per string: up to two 64-row GEMM passes
-constexpr size_t kSmemMax = 227 * 1024;
 
 // rows: connected excitations per GEMM pass (64, or 80 for the FP32 80-row tile,
 // whose Lam_conn rows are 80 elements long)

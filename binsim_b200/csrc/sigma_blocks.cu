@@ -541,8 +541,7 @@ int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, 
     if (!P->ok) return BSIM_OK;
     if (src32) blk_frame_kernel<Ti, float><<<P->v.nAt, 256, 0, s>>>(P->v, B->view.bstrs, src32, P->ct);
     else blk_frame_kernel<Ti, double><<<P->v.nAt, 256, 0, s>>>(P->v, B->view.bstrs, src, P->ct);
-    if (P->smem > 48 * 1024)
-        BSIM_CUDA(cudaFuncSetAttribute(blk_sigma_kernel<Ti>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P->smem));
+    BSIM_CUDA(allow_smem(blk_sigma_kernel<Ti>));
     blk_sigma_kernel<Ti><<<P->v.nAt, kBlkThreads, P->smem, s>>>(P->v, B->view.bstrs, P->ct, dst);
     BSIM_CUDA(cudaGetLastError());
     if (P->n_resid_chunks > 0) {

@@ -1206,7 +1206,7 @@ static int launch_mixed_shape(const DevBasis<Ti> *B, FastPlan<Ti> &P, const Mixe
     constexpr int NT = sizeof(T) == 8 ? 512 : 256;
     constexpr int ROWS = sizeof(T) == 8 ? 64 : (NT / 32) * EPT;
     auto kern = mixed_gemm_kernel<Ti, T, EPT, STREAM, GROW>;
-    BSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BSIM_CUDA(allow_smem(kern));
     const int passes = (P.M + ROWS - 1) / ROWS;   // ROWS connected excitations per GEMM pass
     for (int z0 = c0; z0 < c1; z0 += (int)Wz) {
         for (int pass = 0; pass < passes; ++pass)
@@ -1339,7 +1339,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
             const size_t smem = mixed_dmma_smem(P.ldA, P.nF, !on_chip);
             if (smem <= kSmemMax) {
                 auto kern = on_chip ? mixed_dmma_kernel<Ti, false> : mixed_dmma_kernel<Ti, true>;
-                BSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                BSIM_CUDA(allow_smem(kern));
                 const int passes = (P.M + 63) / 64;
                 T *Z = static_cast<T *>(z.p);
                 const size_t Wz = z.w;
@@ -1398,7 +1398,7 @@ static int launch_ri(const RISide &R, const T *in, int ld_in, double *out, int l
     RIArgs ra{R.nM, R.nU, R.npr, R.nP, ld_in, c1, R.src, R.pid,
               sizeof(T) == 8 ? (const void *)R.W : (const void *)R.W32};
     const size_t smem = ri_smem_bytes(R.nU, sizeof(T));
-    BSIM_CUDA(cudaFuncSetAttribute(ri_gemm_kernel<T, EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BSIM_CUDA(allow_smem(ri_gemm_kernel<T, EPT>));
     T *Z = static_cast<T *>(z.p);
     if constexpr (sizeof(T) == 8) {
         // FP64: per-warp B fragments, all rows on the DMMA path (measured per
@@ -1406,7 +1406,7 @@ static int launch_ri(const RISide &R, const T *in, int ld_in, double *out, int l
         // the shared-slice kernel)
         if (ri_dmma_on() && R.nU <= kRiMaxU && ri_dmma_smem(R.nU) <= kSmemMax) {
             const size_t sm = ri_dmma_smem(R.nU);
-            BSIM_CUDA(cudaFuncSetAttribute(ri_dmma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            BSIM_CUDA(allow_smem(ri_dmma_kernel));
             for (int z0 = c0; z0 < c1; z0 += (int)Wz) {
                 STAGE(tm, 7, s, (launch_chained(ri_dmma_kernel, R.nM, 512, sm, s, ra, in, Z, z0, (int)Wz)));
                 dim3 g(nrows, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));

@@ -609,7 +609,7 @@ int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, const double *ct, cons
 {
     const size_t smem = split_layout(ma.nF, std::min(rows, ma.M - jbase), kMixTab).total;
     auto kern = mixed_gemm_split_kernel<Ti>;
-    BSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BSIM_CUDA(allow_smem(kern));
     launch_chained(kern, ma.nA, kThreads, smem, s, ma, astr, words(ct), rexp, Z, z0, W, jbase, rows);
     BSIM_CUDA(cudaGetLastError());
     return BSIM_OK;

@@ -663,7 +663,7 @@ int mixed_gemm_tc(const MixedArgs &ma, const Ti *astr, const float *ct, float *Z
 {
     const size_t smem = mixed_layout(ma.ldA, ma.nF, N, grow).total;
     auto launch = [&](auto kern) -> int {
-        BSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        BSIM_CUDA(allow_smem(kern));
         kern<<<ma.nA, kTcThreads, smem, s>>>(ma, astr, ct, Z, z0, W, jbase);
         BSIM_CUDA(cudaGetLastError());
         return BSIM_OK;
@@ -685,7 +685,7 @@ int ri_gemm_tc(const RIArgs &ra, const float *in, float *Z, int z0, int W, cudaS
     }
     const size_t smem = ri_layout(ra.nU).total;
     auto launch = [&](auto kern) -> int {
-        BSIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        BSIM_CUDA(allow_smem(kern));
         kern<<<ra.nM, kTcThreads, smem, s>>>(ra, in, Z, z0, W);
         BSIM_CUDA(cudaGetLastError());
         return BSIM_OK;

@@ -89,3 +89,32 @@ def test_bases_in_turn_make_no_new_plans(cuda):
     n = lib().bsim_device_alloc_count()
     both()
     assert lib().bsim_device_alloc_count() == n
+
+
+def test_shapes_of_two_threads(cuda):
+    """Kernels launched with one thread's shared memory while another launches them with less (or more)."""
+    from binsim_b200 import cuotf, network as nw
+    errors = []
+    sizes = ((8, 3, 4), (11, 4, 3))
+    fs = [cuotf.CuOTFFunctions(cuotf.CuBasis(*n), cuotf.CuNetwork(nw.hamiltonian_network(n[0], seed=1, native=True)))
+          for n in sizes]
+
+    def run(f):
+        try:
+            stream = cuda.cuda.Stream()
+            with cuda.cuda.stream(stream):
+                x = cuda.randn(f.basis.dim, dtype=cuda.float64, device="cuda")
+                y = cuda.empty_like(x)
+                for _ in range(300):
+                    f.hvec(x, y)
+                    f.hvec_mixed(x, y)
+                stream.synchronize()
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(f,)) for f in fs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors

@@ -518,8 +518,13 @@ int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, 
 {
     *used = false;
     if (B->num_blocks < 2) return BSIM_OK;
-    std::shared_ptr<BlkPlan<Ti>> P;
-    const int st = N->blk_plans.get(B->serial, &P, [&](std::shared_ptr<BlkPlan<Ti>> &plan) {
+    std::shared_ptr<BlkPlan<Ti>> P = N->blk_plans.template find<BlkPlan<Ti>>(B->serial);
+    if (!P) {   // making the lists allocates and waits: not inside a capture, whose call the tile kernel serves
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        BSIM_CUDA(cudaStreamIsCapturing(s, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return BSIM_OK;
+    }
+    const int st = P ? BSIM_OK : N->blk_plans.get(B->serial, &P, [&](std::shared_ptr<BlkPlan<Ti>> &plan) {
         auto p = std::make_shared<BlkPlan<Ti>>();
         int rc = build(B, N, p.get());
         if (rc == BSIM_OK && p->ok) {

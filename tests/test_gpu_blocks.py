@@ -61,3 +61,30 @@ def test_blocked_sigma_with_other_groups(cuda, oracle):
     y = cuda.empty(B.dim, dtype=cuda.float64, device="cuda")
     f.hvec(dev(cuda, x), y)
     assert np.abs(y.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+def test_first_call_inside_a_capture(cuda, oracle):
+    """The first sigma inside a stream capture takes the tile kernel, which makes nothing (its tile table comes from the
+    diagonal); the captured graph stays good after later calls have made the lists."""
+    from binsim_b200 import cuotf
+    norb, sym = 6, np.array([0, 1, 0, 1, 1, 0], np.int64)
+    net = _masked(norb, sym, 3)
+    kw = dict(orbsym=sym, num_irreps=2)
+    Bo, No = oracle.basis(norb, 3, 2, **kw), oracle.network(net)
+    B = cuotf.CuBasis(norb, 3, 2, **kw)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+    x = np.random.default_rng(2).normal(size=B.dim)
+    ref = oracle.hvec(Bo, No, x)
+    f.get_diags(cuda.zeros(B.dim, dtype=cuda.float64, device="cuda"))
+    xd = dev(cuda, x)
+    y, z = cuda.zeros_like(xd), cuda.zeros_like(xd)
+    s = cuda.cuda.Stream()
+    with cuda.cuda.stream(s):
+        g = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(g, stream=s):
+            f.hvec(xd, y, stream=s.cuda_stream)
+    f.hvec(xd, z)
+    g.replay()
+    cuda.cuda.synchronize()
+    for out in (y, z):
+        assert np.abs(out.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()

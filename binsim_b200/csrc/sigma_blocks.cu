@@ -203,59 +203,252 @@ u64 mask_above_odd(u64 x, int norb)   // orbitals with an odd number of x bits a
     return m;
 }
 
+// ---- the lists, made on the device -----------------------------------------------------
+// The host sorts the groups into forms; a warp per string finds the string's partners
+// by its index tables, first to count its entries, then to write them in the order of
+// the groups.  At 14o 7a+7b in eight irreps the first sigma takes 2.7 ms with them;
+// with lists made by the host it took 105 ms, and through the tile kernel 5.1 ms.
+
+// a pure group: own-spin flip mask, masks and weights; first row of its table of
+// other-spin factors, or -1 and the constant factors
+struct PureG {
+    u64 x;
+    i64 zo, wo;
+    int nz, rank, tab, pad;
+    double c[kSideMaxRank];
+};
+// a row of a factor table: masks and weights of the other spin, the frame's mask
+struct TabG {
+    i64 zo, wo;
+    u64 cm;
+    int nz, r;
+};
+// an excitation of one spin: flipped orbitals, sign mask, irrep
+struct ExcG {
+    u64 x, m;
+    int irr, pad;
+};
+
 template <typename Ti>
-int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
+__device__ __forceinline__ double blk_phase(const NetView<Ti> &N, u64 s, i64 zo, i64 wo, int nz, int r, u64 zxor)
+{
+    double v = 0.0;
+    for (int q = 0; q < nz; ++q) {
+        const double x = N.w[wo + (i64)r * nz + q];
+        v += par(s & ((u64)N.z[zo + q] ^ zxor)) ? -x : x;
+    }
+    return v;
+}
+// block of a string's index in the list of all blocks' strings
+__device__ __forceinline__ int blk_of(const int *start, int nblk, int i)
+{
+    int k = 0;
+    while (k + 1 < nblk && start[k + 1] <= i) ++k;
+    return k;
+}
+// place of string t in block k, or -1
+template <typename Ti>
+__device__ __forceinline__ int blk_find(const BasisView<Ti> &B, bool beta, int k, u64 t)
+{
+    const int loc = string_index(B, beta ? B.bmap : B.amap, beta ? B.nel_b : B.nel_a, (Ti)t);
+    if (loc < 0 || loc >= (beta ? B.blk_nb : B.blk_na)[k]) return -1;
+    const int i = (beta ? B.blk_bstart : B.blk_astart)[k] + loc;
+    return (u64)(beta ? B.bstrs : B.astrs)[i] == t ? loc : -1;
+}
+
+// per row: its block, frame mask and diagonal factors; per column: its diagonal factors
+template <typename Ti>
+__global__ void blk_strings_kernel(const BasisView<Ti> B, const NetView<Ti> N, int diag, int nAt, int nBt,
+                                   int *__restrict__ row_blk, u64 *__restrict__ Ka, double *__restrict__ PAd,
+                                   double *__restrict__ PBd)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    GroupDev g{};
+    if (diag >= 0) g = N.g[diag];
+    if (i < nAt) {
+        const u64 s = (u64)B.astrs[i];
+        u64 K = 0;
+        for (u64 y = s; y; y &= y - 1) K ^= (y & (~y + 1)) - 1;
+        row_blk[i] = blk_of(B.blk_astart, B.num_blocks, i);
+        Ka[i] = K;
+        for (int r = 0; r < g.rank; ++r) PAd[(i64)i * g.rank + r] = blk_phase(N, s, g.za_off, g.wa_off, g.nza, r, 0);
+    } else if (i < nAt + nBt) {
+        const int b = i - nAt;
+        for (int r = 0; r < g.rank; ++r)
+            PBd[(i64)r * nBt + b] = blk_phase(N, (u64)B.bstrs[b], g.zb_off, g.wb_off, g.nzb, r, 0);
+    }
+}
+
+// factor tables: entry (row t, string s) at t * rs + s * ss
+template <typename Ti>
+__global__ void blk_tab_kernel(const NetView<Ti> N, const Ti *__restrict__ strs, int n, const TabG *__restrict__ tabs,
+                               i64 rs, i64 ss, double *__restrict__ out)
+{
+    const TabG t = tabs[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        out[(i64)blockIdx.y * rs + (i64)i * ss] = blk_phase(N, (u64)strs[i], t.zo, t.wo, t.nz, t.r, t.cm);
+}
+
+template <typename Ti>
+__global__ void blk_gidx_kernel(const BasisView<Ti> B, int nBt, const ExcG *__restrict__ F, int *__restrict__ gidx)
+{
+    const ExcG f = F[blockIdx.y];
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nBt; b += gridDim.x * blockDim.x) {
+        const u64 s = (u64)B.bstrs[b], t = s ^ f.x;
+        int g = -1;
+        if (__popcll(s & f.x) == 1) {
+            const int loc = string_index(B, B.bmap, B.nel_b, (Ti)t);
+            if (loc >= 0) g = (loc << 1) | par(t & f.m);
+        }
+        gidx[(i64)blockIdx.y * nBt + b] = g;
+    }
+}
+
+constexpr int kBuildWarps = 8;
+
+// Connected alpha singles of every row, E sorted by irrep; out == nullptr: counts per
+// irrep (zeroed before) into cnt[row][nirr], else entries from ep[row][0].
+template <typename Ti>
+__global__ void __launch_bounds__(32 * kBuildWarps)
+blk_singles_kernel(const BasisView<Ti> B, int nAt, int nirr, int nE, const ExcG *__restrict__ E, int *__restrict__ cnt,
+                   const int *__restrict__ ep, BExc *__restrict__ out)
+{
+    const int a = blockIdx.x * kBuildWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (a >= nAt) return;
+    const u64 s = (u64)B.astrs[a];
+    const int asym = B.blk_asym[blk_of(B.blk_astart, B.num_blocks, a)];
+    int at = out ? ep[(i64)a * (nirr + 1)] : 0;
+    for (int e0 = 0; e0 < nE; e0 += 32) {
+        const int e = e0 + lane;
+        int ks = -1, loc = -1;
+        ExcG x{};
+        if (e < nE && __popcll(s & (x = E[e]).x) == 1) {
+            for (int k = 0; k < B.num_blocks; ++k)
+                if (B.blk_asym[k] == (asym ^ x.irr)) ks = k;
+            if (ks >= 0) loc = blk_find(B, false, ks, s ^ x.x);
+        }
+        const unsigned on = __ballot_sync(0xffffffffu, loc >= 0);
+        if (loc >= 0) {
+            if (out)
+                out[at + __popc(on & ((1u << lane) - 1))] =
+                    BExc{B.blk_off[ks] + (i64)loc * B.blk_nb[ks], (e << 1) | par((s ^ x.x) & x.m), 0};
+            else
+                atomicAdd(cnt + (i64)a * nirr + x.irr, 1);
+        }
+        at += __popc(on);
+    }
+}
+
+// where the entries of one spin's strings go: rows of alpha strings by CSR, beta
+// columns by entry (BlkView)
+struct PureOut {
+    const i64 *acp, *atp;
+    BEnt *ac;
+    BTab *at;
+    int nBt;
+    int *bcs, *bts, *btt;
+    double *bcc, *btp;
+};
+
+// Pure entries of every string of one spin; W.ac == W.bcs == nullptr: counts of
+// constant and table entries into cnt[string].
+template <typename Ti, bool BETA, bool COUNT>
+__global__ void __launch_bounds__(32 * kBuildWarps)
+blk_pure_kernel(const BasisView<Ti> B, const NetView<Ti> N, int n, int ng, const PureG *__restrict__ G,
+                int2 *__restrict__ cnt, const PureOut W)
+{
+    const int i = blockIdx.x * kBuildWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= n) return;
+    const u64 s = (u64)(BETA ? B.bstrs : B.astrs)[i];
+    const int k = blk_of(BETA ? B.blk_bstart : B.blk_astart, B.num_blocks, i);
+    int nc = 0, nt = 0;
+    for (int q0 = 0; q0 < ng; q0 += 32) {
+        const int q = q0 + lane;
+        int loc = -1, tab = 0;
+        u64 x = 0;
+        if (q < ng) {
+            x = G[q].x;
+            tab = G[q].tab;
+            if (2 * __popcll(s & x) == __popcll(x)) loc = blk_find(B, BETA, k, s ^ x);
+        }
+        const unsigned c = __ballot_sync(0xffffffffu, loc >= 0 && tab < 0);
+        const unsigned t = __ballot_sync(0xffffffffu, loc >= 0 && tab >= 0);
+        if (!COUNT && loc >= 0) {
+            const PureG g = G[q];
+            const int pos = tab < 0 ? nc + __popc(c & ((1u << lane) - 1)) : nt + __popc(t & ((1u << lane) - 1));
+            const i64 src = BETA ? loc : B.blk_off[k] + (i64)loc * B.blk_nb[k];
+            double p[kSideMaxRank] = {0.0, 0.0, 0.0, 0.0}, coef = 0.0;
+            for (int r = 0; r < g.rank; ++r) {
+                p[r] = blk_phase(N, s ^ x, g.zo, g.wo, g.nz, r, 0);
+                coef += p[r] * g.c[r];
+            }
+            if (BETA) {
+                const i64 o = (i64)pos * W.nBt + i;
+                if (tab < 0) {
+                    W.bcs[o] = (int)src;
+                    W.bcc[o] = coef;
+                } else {
+                    W.bts[o] = (int)src;
+                    W.btt[o] = (tab << 3) | g.rank;
+                    for (int r = 0; r < kSideMaxRank; ++r) W.btp[((i64)pos * kSideMaxRank + r) * W.nBt + i] = p[r];
+                }
+            } else if (tab < 0) {
+                W.ac[W.acp[i] + pos] = BEnt{src, coef};
+            } else {
+                W.at[W.atp[i] + pos] = BTab{src, (tab << 3) | g.rank, 0, {p[0], p[1], p[2], p[3]}};
+            }
+        }
+        nc += __popc(c);
+        nt += __popc(t);
+    }
+    if (COUNT && lane == 0) cnt[i] = make_int2(nc, nt);
+}
+
+// pieces of one device allocation
+struct Blob {
+    size_t n = 0;
+    template <typename T>
+    size_t add(size_t count)
+    {
+        const size_t o = (n + 255) & ~size_t(255);
+        n = o + std::max<size_t>(count, 1) * sizeof(T);
+        return o;
+    }
+};
+struct TempMem {
+    char *p = nullptr;
+    ~TempMem() { if (p) cudaFree(p); }
+};
+
+template <typename Ti>
+int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P, cudaStream_t s)
 {
     P->ok = false;
     const int norb = B->norb, nirr = B->num_irreps;
     if (B->num_blocks < 2 || norb > 63 || N->norb > norb || N->cplx) return BSIM_OK;
     const u64 full = (1ull << norb) - 1;
     const int nAt = (int)B->astrs.size(), nBt = (int)B->bstrs.size();
-    // string -> block, local index, per spin
-    struct Where { int blk, loc; };
-    auto index = [&](const std::vector<Ti> &strs, const std::vector<int> &start, const std::vector<int> &cnt) {
-        std::unordered_map<u64, Where> m;
-        m.reserve(strs.size() * 2);
-        for (int k = 0; k < B->num_blocks; ++k)
-            for (int i = 0; i < cnt[k]; ++i) m[(u64)strs[start[k] + i]] = Where{k, i};
-        return m;
-    };
-    const auto amap = index(B->astrs, B->astart, B->na), bmap = index(B->bstrs, B->bstart, B->nb);
-    std::vector<int> row_blk(nAt), col_blk(nBt);
-    std::vector<u64> Ka(nAt);
-    for (int k = 0; k < B->num_blocks; ++k) {
-        for (int i = 0; i < B->na[k]; ++i) row_blk[B->astart[k] + i] = k;
-        for (int i = 0; i < B->nb[k]; ++i) col_blk[B->bstart[k] + i] = k;
-    }
-    for (int a = 0; a < nAt; ++a)
-        for (int i = 0; i < norb; ++i)
-            if (((u64)B->astrs[a] >> i) & 1u) Ka[a] ^= (1ull << i) - 1;
     const Ti *z = N->z.data();
     const double *w = N->w.data();
-    auto phase = [&](u64 s, i64 zo, i64 wo, int nz, int r, u64 zxor) {
+    auto phase = [&](u64 x, i64 zo, i64 wo, int nz, int r, u64 zxor) {
         double v = 0.0;
         for (int q = 0; q < nz; ++q) {
-            const double x = w[wo + (i64)r * nz + q];
-            v += (popc(s & ((u64)z[zo + q] ^ zxor)) & 1) ? -x : x;
+            const double y = w[wo + (i64)r * nz + q];
+            v += (popc(x & ((u64)z[zo + q] ^ zxor)) & 1) ? -y : y;
         }
         return v;
     };
 
     std::vector<int> residual;
-    std::vector<double> PAd, PBd;
     int rank_d = 0, diag = -1;
-    // pure groups of one spin: own masks and weights, other-spin factor constant or tabled
-    struct Side {
-        std::vector<int> g, tab;              // group, first table row or -1
-        std::vector<double> c;                // constant factors [kSideMaxRank]
-        std::vector<double> tabs;             // [rows][other strings]
-        int nt = 0;
+    struct Side {   // pure groups of one spin, their tables of other-spin factors
+        std::vector<PureG> g;
+        std::vector<TabG> tabs;
     } sd[2];
     struct Rec { int E, F; double v; };
     std::vector<Rec> recs;
     std::unordered_map<u64, int> eid, fid;
-    std::vector<u64> Em, Fm, mA, mB;
-    std::vector<int> Firr, Eirr;
+    std::vector<ExcG> Eg, Fg;
     for (i64 gi = 0; gi < N->ngs; ++gi) {
         const GroupDev &G = N->groups[(size_t)gi];
         if (G.rank == 0) continue;
@@ -264,12 +457,6 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
             if (diag >= 0) { residual.push_back((int)gi); continue; }
             diag = (int)gi;
             rank_d = G.rank;
-            PAd.resize((size_t)nAt * rank_d);
-            PBd.resize((size_t)nBt * rank_d);
-            for (int r = 0; r < rank_d; ++r) {
-                for (int a = 0; a < nAt; ++a) PAd[(size_t)a * rank_d + r] = phase((u64)B->astrs[a], G.za_off, G.wa_off, G.nza, r, 0);
-                for (int b = 0; b < nBt; ++b) PBd[(size_t)r * nBt + b] = phase((u64)B->bstrs[b], G.zb_off, G.wb_off, G.nzb, r, 0);
-            }
         } else if (G.type == 1 || G.type == 2) {
             if (G.rank > kSideMaxRank) { residual.push_back((int)gi); continue; }
             Side &S = sd[G.type - 1];
@@ -277,21 +464,19 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
             const u64 cm = al ? mask_above_odd(G.ax, norb) : mask_below_odd(G.bx, norb);
             const i64 zo = al ? G.zb_off : G.za_off, wo = al ? G.wb_off : G.wa_off;
             const int nz = al ? G.nzb : G.nza;
-            const auto &other = al ? B->bstrs : B->astrs;
+            const u64 other = (u64)(al ? B->bstrs : B->astrs)[0];
             bool constant = true;             // every mask empty or full in the frame
             for (int q = 0; q < nz; ++q) {
                 const u64 m = ((u64)z[zo + q] ^ cm) & full;
                 if (m != 0 && m != full) constant = false;
             }
-            S.g.push_back((int)gi);
-            S.tab.push_back(constant ? -1 : S.nt);
-            for (int r = 0; r < kSideMaxRank; ++r)
-                S.c.push_back(constant && r < G.rank ? phase((u64)other[0], zo, wo, nz, r, cm) : 0.0);
-            if (!constant) {
-                for (int r = 0; r < G.rank; ++r)
-                    for (size_t s = 0; s < other.size(); ++s) S.tabs.push_back(phase((u64)other[s], zo, wo, nz, r, cm));
-                S.nt += G.rank;
+            PureG p{al ? G.ax : G.bx, al ? G.za_off : G.zb_off, al ? G.wa_off : G.wb_off, al ? G.nza : G.nzb, G.rank,
+                    constant ? -1 : (int)S.tabs.size(), 0, {0.0, 0.0, 0.0, 0.0}};
+            for (int r = 0; r < G.rank; ++r) {
+                if (constant) p.c[r] = phase(other, zo, wo, nz, r, cm);
+                else S.tabs.push_back(TabG{zo, wo, cm, nz, r});
             }
+            S.g.push_back(p);
         } else {
             if (G.rank != 1 || popc(G.ax) != 2 || popc(G.bx) != 2) { residual.push_back((int)gi); continue; }
             const u64 ma = mask_below_odd(G.bx, norb), mb = mask_above_odd(G.ax, norb);
@@ -303,18 +488,18 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
                     if ((((u64)z[zo + q] ^ zx ^ m) & full & ~x) != 0) return false;
                 const u64 p = x & (~x + 1), q = x ^ p;
                 double v[2];
-                const u64 s[2] = {p, q};
+                const u64 one[2] = {p, q};
                 for (int i = 0; i < 2; ++i) {
-                    v[i] = phase(s[i], zo, wo, nz, 0, zx);
-                    if (popc(s[i] & m) & 1) v[i] = -v[i];
+                    v[i] = phase(one[i], zo, wo, nz, 0, zx);
+                    if (popc(one[i] & m) & 1) v[i] = -v[i];
                 }
                 *out = v[0];
                 return std::fabs(v[0] - v[1]) <= 1e-12 * std::max(1.0, std::fabs(v[0]));
             };
             const auto ei = eid.find(G.ax);
             const auto fi = fid.find(G.bx);
-            const u64 sa = ei == eid.end() ? (u64)z[G.za_off] ^ ma : mA[ei->second];
-            const u64 sb = fi == fid.end() ? (u64)z[G.zb_off] ^ mb : mB[fi->second];
+            const u64 sa = ei == eid.end() ? (u64)z[G.za_off] ^ ma : Eg[ei->second].m;
+            const u64 sb = fi == fid.end() ? (u64)z[G.zb_off] ^ mb : Fg[fi->second].m;
             double lam, mu;
             if (G.nza < 1 || G.nzb < 1 || !factor(G.ax, G.za_off, G.wa_off, G.nza, ma, sa, &lam) ||
                 !factor(G.bx, G.zb_off, G.wb_off, G.nzb, mb, sb, &mu)) {
@@ -323,138 +508,40 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
             }
             int E = ei == eid.end() ? -1 : ei->second, F = fi == fid.end() ? -1 : fi->second;
             if (E < 0) {
-                E = (int)Em.size();
+                E = (int)Eg.size();
                 eid[G.ax] = E;
-                Em.push_back(G.ax);
-                mA.push_back(sa);
-                Eirr.push_back(G.asym);
+                Eg.push_back(ExcG{G.ax, sa, G.asym, 0});
             }
             if (F < 0) {
-                F = (int)Fm.size();
+                F = (int)Fg.size();
                 fid[G.bx] = F;
-                Fm.push_back(G.bx);
-                mB.push_back(sb);
-                Firr.push_back(G.bsym);
+                Fg.push_back(ExcG{G.bx, sb, G.bsym, 0});
             }
             recs.push_back({E, F, ((popc(G.ax & ma) & 1) ? -1.0 : 1.0) * lam * mu});
         }
     }
-    const int nE = (int)Em.size(), nF = (int)Fm.size();
-    // F sorted by irrep
-    std::vector<int> forder(nF), fpos(nF), fp(nirr + 1, 0);
-    for (int f = 0; f < nF; ++f) forder[f] = f;
-    std::stable_sort(forder.begin(), forder.end(), [&](int x, int y) { return Firr[x] < Firr[y]; });
-    for (int i = 0; i < nF; ++i) {
-        fpos[forder[i]] = i;
-        if (Firr[forder[i]] >= nirr) return BSIM_OK;
-        ++fp[Firr[forder[i]] + 1];
-    }
+    const int nE = (int)Eg.size(), nF = (int)Fg.size(), nt0 = (int)sd[0].tabs.size(), nt1 = (int)sd[1].tabs.size();
+    if (nt0 > 65535 || nt1 > 65535) return BSIM_OK;   // a grid dimension of blk_tab_kernel
+    // E and F sorted by irrep
+    auto by_irrep = [&](std::vector<ExcG> &v, std::vector<int> &pos) {
+        std::vector<int> order(v.size());
+        for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return v[x].irr < v[y].irr; });
+        std::vector<ExcG> t(v.size());
+        pos.resize(v.size());
+        for (size_t i = 0; i < order.size(); ++i) {
+            t[i] = v[order[i]];
+            pos[order[i]] = (int)i;
+        }
+        v.swap(t);
+        return v.empty() || v.back().irr < nirr;
+    };
+    std::vector<int> epos, fpos, fp(nirr + 1, 0);
+    if (!by_irrep(Eg, epos) || !by_irrep(Fg, fpos)) return BSIM_OK;
+    for (const ExcG &f : Fg) ++fp[f.irr + 1];
     for (int g = 0; g < nirr; ++g) fp[g + 1] += fp[g];
     std::vector<double> Lam((size_t)nE * nF, 0.0);
-    for (const Rec &r : recs) Lam[(size_t)r.E * nF + fpos[r.F]] += r.v;
-    std::vector<int> gidx((size_t)nF * nBt, -1);
-    for (int i = 0; i < nF; ++i) {
-        const u64 fm = Fm[forder[i]], sm = mB[forder[i]];
-        for (int b = 0; b < nBt; ++b) {
-            const u64 s = (u64)B->bstrs[b];
-            if (popc(s & fm) != 1) continue;
-            const auto it = bmap.find(s ^ fm);
-            if (it != bmap.end()) gidx[(size_t)i * nBt + b] = (it->second.loc << 1) | (popc((s ^ fm) & sm) & 1);
-        }
-    }
-    // connected alpha singles per row, by irrep, where the source block exists
-    std::vector<int> ep((size_t)nAt * (nirr + 1), 0);
-    std::vector<BExc> ex;
-    std::vector<int> eorder(nE);
-    for (int e = 0; e < nE; ++e) eorder[e] = e;
-    std::stable_sort(eorder.begin(), eorder.end(), [&](int x, int y) { return Eirr[x] < Eirr[y]; });
-    size_t lam_max = 0;
-    for (int a = 0; a < nAt; ++a) {
-        const u64 s = (u64)B->astrs[a];
-        int *p = &ep[(size_t)a * (nirr + 1)];
-        size_t nl = 0, i = 0;
-        for (int g = 0; g < nirr; ++g) {
-            p[g] = (int)ex.size();
-            for (; i < eorder.size() && Eirr[eorder[i]] <= g; ++i) {
-                const int e = eorder[i];
-                if (popc(s & Em[e]) != 1) continue;
-                const auto it = amap.find(s ^ Em[e]);
-                if (it == amap.end()) continue;
-                const int ks = it->second.blk;
-                ex.push_back(BExc{B->off[ks] + (i64)it->second.loc * B->nb[ks], (e << 1) | (popc((s ^ Em[e]) & mA[e]) & 1), 0});
-            }
-            nl += (size_t)((int)ex.size() - p[g]) * (fp[g + 1] - fp[g]);
-        }
-        p[nirr] = (int)ex.size();
-        lam_max = std::max(lam_max, nl);
-    }
-    if (ex.size() > ((size_t)1 << 30)) return BSIM_OK;
-    // pure entries of every alpha row and of every beta column
-    std::vector<i64> cp[2], tp[2];
-    std::vector<BEnt> ce[2];
-    std::vector<BTab> te[2];
-    for (int side = 0; side < 2; ++side) {
-        const Side &S = sd[side];
-        const auto &strs = side == 0 ? B->astrs : B->bstrs;
-        const auto &map = side == 0 ? amap : bmap;
-        const auto &blk = side == 0 ? row_blk : col_blk;
-        cp[side].assign(1, 0);
-        tp[side].assign(1, 0);
-        for (size_t i = 0; i < strs.size(); ++i) {
-            const u64 s = (u64)strs[i];
-            for (size_t q = 0; q < S.g.size(); ++q) {
-                const GroupDev &G = N->groups[(size_t)S.g[q]];
-                const u64 x = side == 0 ? G.ax : G.bx;
-                if (2 * popc(s & x) != popc(x)) continue;
-                const auto it = map.find(s ^ x);
-                if (it == map.end() || it->second.blk != blk[i]) continue;
-                const i64 zo = side == 0 ? G.za_off : G.zb_off, wo = side == 0 ? G.wa_off : G.wb_off;
-                const int nz = side == 0 ? G.nza : G.nzb, k = it->second.blk;
-                const long long src = side == 0 ? B->off[k] + (i64)it->second.loc * B->nb[k] : it->second.loc;
-                double p[kSideMaxRank] = {0, 0, 0, 0}, c = 0.0;
-                for (int r = 0; r < G.rank; ++r) {
-                    p[r] = phase(s ^ x, zo, wo, nz, r, 0);
-                    c += p[r] * S.c[q * kSideMaxRank + r];
-                }
-                if (S.tab[q] < 0) ce[side].push_back(BEnt{src, c});
-                else te[side].push_back(BTab{src, (S.tab[q] << 3) | G.rank, 0, {p[0], p[1], p[2], p[3]}});
-            }
-            cp[side].push_back((i64)ce[side].size());
-            tp[side].push_back((i64)te[side].size());
-        }
-    }
-    size_t max_ac = 0, max_ex = 0, nbc = 0, nbt = 0;
-    for (int a = 0; a < nAt; ++a) {
-        max_ac = std::max(max_ac, (size_t)(cp[0][a + 1] - cp[0][a]));
-        max_ex = std::max(max_ex, (size_t)(ep[(size_t)a * (nirr + 1) + nirr] - ep[(size_t)a * (nirr + 1)]));
-    }
-    for (int b = 0; b < nBt; ++b) {
-        nbc = std::max(nbc, (size_t)(cp[1][b + 1] - cp[1][b]));
-        nbt = std::max(nbt, (size_t)(tp[1][b + 1] - tp[1][b]));
-    }
-    P->smem = (lam_max + (size_t)sd[1].nt + 2 * max_ac + max_ex) * sizeof(double);
-    if (P->smem > kBlkSmem) return BSIM_OK;
-    // the beta entries by column
-    std::vector<int> bcs(nbc * nBt, -1), bts(nbt * nBt, -1), btt(nbt * nBt, 0);
-    std::vector<double> bcc(nbc * nBt, 0.0), btp(nbt * kSideMaxRank * nBt, 0.0);
-    for (int b = 0; b < nBt; ++b) {
-        for (i64 i = cp[1][b]; i < cp[1][b + 1]; ++i) {
-            const size_t o = (size_t)(i - cp[1][b]) * nBt + b;
-            bcs[o] = (int)ce[1][(size_t)i].src;
-            bcc[o] = ce[1][(size_t)i].coef;
-        }
-        for (i64 i = tp[1][b]; i < tp[1][b + 1]; ++i) {
-            const size_t e = (size_t)(i - tp[1][b]);
-            const BTab &t = te[1][(size_t)i];
-            bts[e * nBt + b] = (int)t.src;
-            btt[e * nBt + b] = t.t;
-            for (int r = 0; r < kSideMaxRank; ++r) btp[(e * kSideMaxRank + r) * nBt + b] = t.p[r];
-        }
-    }
-    // factors of beta entries by alpha row
-    std::vector<double> tabA((size_t)nAt * sd[1].nt);
-    for (int t = 0; t < sd[1].nt; ++t)
-        for (int a = 0; a < nAt; ++a) tabA[(size_t)a * sd[1].nt + t] = sd[1].tabs[(size_t)t * nAt + a];
+    for (const Rec &r : recs) Lam[(size_t)epos[r.E] * nF + fpos[r.F]] += r.v;
     // residual groups through the tile kernel
     std::stable_sort(residual.begin(), residual.end(), [&](int x, int y) {
         const GroupDev &p = N->groups[x], &q = N->groups[y];
@@ -472,34 +559,120 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P)
         i = j;
     }
 
-    std::vector<char> blob;
-    auto put = [&](const auto &v) {   // offset of the vector in the one upload
-        using T = typename std::decay_t<decltype(v)>::value_type;
-        const size_t o = (blob.size() + 255) & ~size_t(255);
-        blob.resize(o + std::max<size_t>(v.size(), 1) * sizeof(T));
-        if (!v.empty()) memcpy(blob.data() + o, v.data(), v.size() * sizeof(T));
-        return o;
+    // counts
+    auto upload = [](char *d, const auto &v) {
+        return v.empty() ? cudaSuccess : cudaMemcpy(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice);
     };
-    const size_t o_rb = put(row_blk), o_off = put(B->off), o_nb = put(B->nb), o_as = put(B->astart), o_bs = put(B->bstart),
-                 o_Ka = put(Ka), o_PA = put(PAd), o_PB = put(PBd), o_acp = put(cp[0]), o_atp = put(tp[0]),
-                 o_bcs = put(bcs), o_bts = put(bts), o_btt = put(btt), o_bcc = put(bcc), o_btp = put(btp),
-                 o_ac = put(ce[0]), o_at = put(te[0]), o_tB = put(sd[0].tabs), o_tA = put(tabA), o_ep = put(ep), o_ex = put(ex),
-                 o_fp = put(fp), o_L = put(Lam), o_g = put(gidx), o_r = put(residual), o_rc = put(chunks);
-    int st = P->arena.reserve(blob.size());
+    Blob T;
+    const size_t t_g[2] = {T.add<PureG>(sd[0].g.size()), T.add<PureG>(sd[1].g.size())};
+    const size_t t_t[2] = {T.add<TabG>(nt0), T.add<TabG>(nt1)};
+    const size_t t_e = T.add<ExcG>(nE), t_f = T.add<ExcG>(nF);
+    const size_t t_c = T.add<int2>((size_t)nAt + nBt), t_n = T.add<int>((size_t)nAt * nirr);
+    TempMem tmp;
+    cudaError_t e = dmalloc(&tmp.p, T.n);
+    if (e != cudaSuccess) {
+        tmp.p = nullptr;
+        return e == cudaErrorMemoryAllocation ? BSIM_ERR_ALLOC : cuda_status(e, "symmetry-blocked sigma");
+    }
+    for (int side = 0; side < 2; ++side) {
+        BSIM_CUDA(upload(tmp.p + t_g[side], sd[side].g));
+        BSIM_CUDA(upload(tmp.p + t_t[side], sd[side].tabs));
+    }
+    BSIM_CUDA(upload(tmp.p + t_e, Eg));
+    BSIM_CUDA(upload(tmp.p + t_f, Fg));
+    const PureG *dG[2] = {reinterpret_cast<PureG *>(tmp.p + t_g[0]), reinterpret_cast<PureG *>(tmp.p + t_g[1])};
+    const TabG *dT[2] = {reinterpret_cast<TabG *>(tmp.p + t_t[0]), reinterpret_cast<TabG *>(tmp.p + t_t[1])};
+    const ExcG *dE = reinterpret_cast<ExcG *>(tmp.p + t_e), *dF = reinterpret_cast<ExcG *>(tmp.p + t_f);
+    int2 *d_cnt = reinterpret_cast<int2 *>(tmp.p + t_c);
+    int *d_ne = reinterpret_cast<int *>(tmp.p + t_n);
+    const unsigned gA = (unsigned)((nAt + kBuildWarps - 1) / kBuildWarps), gB = (unsigned)((nBt + kBuildWarps - 1) / kBuildWarps);
+    constexpr int kBT = 32 * kBuildWarps;
+    BSIM_CUDA(cudaMemsetAsync(d_ne, 0, sizeof(int) * (size_t)nAt * nirr, s));
+    blk_singles_kernel<Ti><<<gA, kBT, 0, s>>>(B->view, nAt, nirr, nE, dE, d_ne, nullptr, nullptr);
+    blk_pure_kernel<Ti, false, true><<<gA, kBT, 0, s>>>(B->view, N->view, nAt, (int)sd[0].g.size(), dG[0], d_cnt, PureOut{});
+    blk_pure_kernel<Ti, true, true><<<gB, kBT, 0, s>>>(B->view, N->view, nBt, (int)sd[1].g.size(), dG[1], d_cnt + nAt,
+                                                       PureOut{});
+    BSIM_CUDA(cudaGetLastError());
+    std::vector<int2> cnt((size_t)nAt + nBt);
+    std::vector<int> ne((size_t)nAt * nirr);
+    BSIM_CUDA(cudaMemcpyAsync(cnt.data(), d_cnt, cnt.size() * sizeof(int2), cudaMemcpyDeviceToHost, s));
+    BSIM_CUDA(cudaMemcpyAsync(ne.data(), d_ne, ne.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+    BSIM_CUDA(cudaStreamSynchronize(s));
+    std::vector<i64> acp(nAt + 1, 0), atp(nAt + 1, 0);
+    std::vector<int> ep((size_t)nAt * (nirr + 1));
+    i64 nex = 0;
+    size_t max_ac = 0, max_ex = 0, lam_max = 0, nbc = 0, nbt = 0;
+    for (int a = 0; a < nAt; ++a) {
+        acp[a + 1] = acp[a] + cnt[a].x;
+        atp[a + 1] = atp[a] + cnt[a].y;
+        const i64 first = nex;
+        size_t nl = 0;
+        for (int g = 0; g <= nirr; ++g) {
+            ep[(size_t)a * (nirr + 1) + g] = (int)nex;
+            if (g == nirr) break;
+            const int k = ne[(size_t)a * nirr + g];
+            nex += k;
+            nl += (size_t)k * (fp[g + 1] - fp[g]);
+        }
+        if (nex > ((i64)1 << 30)) return BSIM_OK;
+        max_ac = std::max(max_ac, (size_t)cnt[a].x);
+        max_ex = std::max(max_ex, (size_t)(nex - first));
+        lam_max = std::max(lam_max, nl);
+    }
+    for (int b = 0; b < nBt; ++b) {
+        nbc = std::max(nbc, (size_t)cnt[(size_t)nAt + b].x);
+        nbt = std::max(nbt, (size_t)cnt[(size_t)nAt + b].y);
+    }
+    P->smem = (lam_max + (size_t)nt1 + 2 * max_ac + max_ex) * sizeof(double);
+    if (P->smem > kBlkSmem) return BSIM_OK;
+
+    // the lists; what the host made comes first and goes up in one copy
+    Blob D;
+    const size_t o_fp = D.add<int>(nirr + 1), o_L = D.add<double>(Lam.size()), o_acp = D.add<i64>(nAt + 1),
+                 o_atp = D.add<i64>(nAt + 1), o_ep = D.add<int>(ep.size()), o_r = D.add<int>(residual.size()),
+                 o_rc = D.add<int4>(chunks.size());
+    const size_t host_bytes = D.n;
+    const size_t o_rb = D.add<int>(nAt), o_Ka = D.add<u64>(nAt), o_PA = D.add<double>((size_t)nAt * rank_d),
+                 o_PB = D.add<double>((size_t)nBt * rank_d), o_ac = D.add<BEnt>((size_t)acp[nAt]),
+                 o_at = D.add<BTab>((size_t)atp[nAt]), o_bcs = D.add<int>(nbc * nBt), o_bts = D.add<int>(nbt * nBt),
+                 o_btt = D.add<int>(nbt * nBt), o_bcc = D.add<double>(nbc * nBt),
+                 o_btp = D.add<double>(nbt * kSideMaxRank * nBt), o_tB = D.add<double>((size_t)nt0 * nBt),
+                 o_tA = D.add<double>((size_t)nt1 * nAt), o_ex = D.add<BExc>((size_t)nex),
+                 o_g = D.add<int>((size_t)nF * nBt);
+    int st = P->arena.reserve(D.n);
     if (st != BSIM_OK) return st;
-    char *d = P->arena.template take<char>(blob.size());
-    BSIM_CUDA(cudaMemcpy(d, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+    char *d = P->arena.template take<char>(D.n);
+    std::vector<char> host(host_bytes, 0);
+    auto put = [&](size_t o, const auto &v) {
+        if (!v.empty()) memcpy(host.data() + o, v.data(), v.size() * sizeof(v[0]));
+    };
+    put(o_fp, fp); put(o_L, Lam); put(o_acp, acp); put(o_atp, atp); put(o_ep, ep); put(o_r, residual); put(o_rc, chunks);
+    BSIM_CUDA(cudaMemcpy(d, host.data(), host_bytes, cudaMemcpyHostToDevice));
     auto at = [&](auto *type, size_t o) { return reinterpret_cast<decltype(type)>(d + o); };
-    using I = const int *;
-    using L = const i64 *;
-    using D = const double *;
-    P->v = BlkView{nirr, nAt, nBt, rank_d, nF, sd[1].nt, sd[0].nt,
-                   at(I(), o_rb), at(L(), o_off), at(I(), o_nb), at(I(), o_as), at(I(), o_bs),
-                   reinterpret_cast<const u64 *>(d + o_Ka), at(D(), o_PA), at(D(), o_PB), at(L(), o_acp), at(L(), o_atp),
-                   reinterpret_cast<const BEnt *>(d + o_ac), reinterpret_cast<const BTab *>(d + o_at), (int)nbc, (int)nbt,
-                   at(I(), o_bcs), at(I(), o_bts), at(I(), o_btt), at(D(), o_bcc), at(D(), o_btp),
-                   at(D(), o_tB), at(D(), o_tA), at(I(), o_ep),
-                   reinterpret_cast<const BExc *>(d + o_ex), at(I(), o_fp), at(D(), o_L), at(I(), o_g)};
+    using I = int *;
+    using L = i64 *;
+    using R = double *;
+    blk_strings_kernel<Ti><<<(unsigned)((nAt + nBt + 255) / 256), 256, 0, s>>>(
+        B->view, N->view, diag, nAt, nBt, at(I(), o_rb), reinterpret_cast<u64 *>(d + o_Ka), at(R(), o_PA), at(R(), o_PB));
+    const unsigned xB = (unsigned)std::min(256, (nBt + 255) / 256), xA = (unsigned)std::min(256, (nAt + 255) / 256);
+    if (nt0 > 0) blk_tab_kernel<Ti><<<dim3(xB, nt0), 256, 0, s>>>(N->view, B->view.bstrs, nBt, dT[0], nBt, 1, at(R(), o_tB));
+    if (nt1 > 0) blk_tab_kernel<Ti><<<dim3(xA, nt1), 256, 0, s>>>(N->view, B->view.astrs, nAt, dT[1], 1, nt1, at(R(), o_tA));
+    if (nF > 0) blk_gidx_kernel<Ti><<<dim3(xB, nF), 256, 0, s>>>(B->view, nBt, dF, at(I(), o_g));
+    BSIM_CUDA(cudaMemsetAsync(d + o_bcs, 0xff, sizeof(int) * nbc * nBt, s));   // -1: no entry
+    BSIM_CUDA(cudaMemsetAsync(d + o_bts, 0xff, sizeof(int) * nbt * nBt, s));
+    PureOut W{at(L(), o_acp), at(L(), o_atp), reinterpret_cast<BEnt *>(d + o_ac), reinterpret_cast<BTab *>(d + o_at), nBt,
+              at(I(), o_bcs), at(I(), o_bts), at(I(), o_btt), at(R(), o_bcc), at(R(), o_btp)};
+    blk_singles_kernel<Ti><<<gA, kBT, 0, s>>>(B->view, nAt, nirr, nE, dE, nullptr, at(I(), o_ep),
+                                              reinterpret_cast<BExc *>(d + o_ex));
+    blk_pure_kernel<Ti, false, false><<<gA, kBT, 0, s>>>(B->view, N->view, nAt, (int)sd[0].g.size(), dG[0], nullptr, W);
+    blk_pure_kernel<Ti, true, false><<<gB, kBT, 0, s>>>(B->view, N->view, nBt, (int)sd[1].g.size(), dG[1], nullptr, W);
+    BSIM_CUDA(cudaGetLastError());
+    BSIM_CUDA(cudaStreamSynchronize(s));   // the group tables are freed on return
+    P->v = BlkView{nirr, nAt, nBt, rank_d, nF, nt1, nt0,
+                   at(I(), o_rb), B->view.blk_off, B->view.blk_nb, B->view.blk_astart, B->view.blk_bstart,
+                   reinterpret_cast<const u64 *>(d + o_Ka), at(R(), o_PA), at(R(), o_PB), at(L(), o_acp), at(L(), o_atp),
+                   W.ac, W.at, (int)nbc, (int)nbt, W.bcs, W.bts, W.btt, W.bcc, W.btp, at(R(), o_tB), at(R(), o_tA),
+                   at(I(), o_ep), reinterpret_cast<const BExc *>(d + o_ex), at(I(), o_fp), at(R(), o_L), at(I(), o_g)};
     P->d_resid = at(I(), o_r);
     P->d_resid_chunks = reinterpret_cast<const int4 *>(d + o_rc);
     P->n_resid_chunks = (int)chunks.size();
@@ -526,7 +699,7 @@ int sigma_blocks(const DevBasis<Ti> *B, const DevNet<Ti> *N, const double *src, 
     }
     const int st = P ? BSIM_OK : N->blk_plans.get(B->serial, &P, [&](std::shared_ptr<BlkPlan<Ti>> &plan) {
         auto p = std::make_shared<BlkPlan<Ti>>();
-        int rc = build(B, N, p.get());
+        int rc = build(B, N, p.get(), s);
         if (rc == BSIM_OK && p->ok) {
             const cudaError_t e = dmalloc(&p->ct, sizeof(double) * B->dim);
             if (e != cudaSuccess) {

@@ -88,3 +88,28 @@ def test_first_call_inside_a_capture(cuda, oracle):
     cuda.cuda.synchronize()
     for out in (y, z):
         assert np.abs(out.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()
+
+
+def test_first_call_is_no_slower_than_the_tile_kernel(cuda):
+    """What the first call on a handle pays for the lists: compared with one call that needs none (hvec_tiles over every
+    tile).  Made by the host they took twenty times that at this size; three times is the line."""
+    import time
+    from binsim_b200 import cuotf
+    norb, sym = 14, np.array([0, 5, 0, 6, 7, 0, 2, 3, 5, 1, 4, 0, 5, 6], np.int64)
+    net = _masked(norb, sym, 0)
+    B = cuotf.CuBasis(norb, 7, 7, orbsym=sym, num_irreps=8)
+    x = cuda.randn(B.dim, dtype=cuda.float64, device="cuda")
+    y = cuda.empty_like(x)
+
+    def ms(call, *args):
+        cuda.cuda.synchronize()
+        t = time.perf_counter()
+        call(*args)
+        cuda.cuda.synchronize()
+        return 1e3 * (time.perf_counter() - t)
+    first, tiles = [], []
+    for _ in range(4):
+        f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+        first.append(ms(f.hvec, x, y))
+        tiles.append(ms(f.hvec_tiles, x, y, 0, f.num_tiles()))
+    assert min(first[1:]) <= 3.0 * min(tiles[1:]), (first, tiles)

@@ -170,6 +170,9 @@ inline MixedShape mixed_shape(int nB, int nF, size_t elem, size_t row_limit, int
     return MixedShape{true, true, mixed_smem_bytes(nB, nF, elem, true, true, rows)};
 }
 
+// Bytes that a sigma may take for its intermediates (BSIM_SIGMA_SCRATCH_GB).
+size_t scratch_limit();
+
 template <typename Ti>
 int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P);
 

@@ -34,6 +34,7 @@ namespace {
 
 constexpr int kBlkThreads = 128;
 constexpr size_t kBlkSmem = 96 * 1024;    // Lam_conn and the row factors of one row
+constexpr size_t kBlkLists = (size_t)2 << 30;   // larger lists: the tile kernel
 
 // a constant-factor entry of an alpha row: source row (element offset), coefficient
 struct BEnt {
@@ -639,6 +640,12 @@ int build(const DevBasis<Ti> *B, const DevNet<Ti> *N, BlkPlan<Ti> *P, cudaStream
                  o_btp = D.add<double>(nbt * kSideMaxRank * nBt), o_tB = D.add<double>((size_t)nt0 * nBt),
                  o_tA = D.add<double>((size_t)nt1 * nAt), o_ex = D.add<BExc>((size_t)nex),
                  o_g = D.add<int>((size_t)nF * nBt);
+    // The tile kernel needs no memory: it serves where the lists would be larger than
+    // kBlkLists (14o 7a+7b in eight irreps takes 18 MB, 16o 8a+8b 90 MB), or lists and
+    // frame vector larger than sigma's scratch limit or half of the free memory.
+    size_t free_b = 0, total_b = 0;
+    BSIM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (D.n > kBlkLists || D.n + sizeof(double) * (size_t)B->dim > std::min(scratch_limit(), free_b / 2)) return BSIM_OK;
     int st = P->arena.reserve(D.n);
     if (st != BSIM_OK) return st;
     char *d = P->arena.template take<char>(D.n);

@@ -1089,7 +1089,7 @@ static int get_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, std::shared_ptr<
     });
 }
 
-static size_t scratch_limit()
+size_t scratch_limit()
 {
     const char *e = getenv("BSIM_SIGMA_SCRATCH_GB");
     double gb = e ? atof(e) : 24.0;

@@ -113,3 +113,36 @@ def test_first_call_is_no_slower_than_the_tile_kernel(cuda):
         first.append(ms(f.hvec, x, y))
         tiles.append(ms(f.hvec_tiles, x, y, 0, f.num_tiles()))
     assert min(first[1:]) <= 3.0 * min(tiles[1:]), (first, tiles)
+
+
+def test_lists_stay_within_the_scratch_limit(cuda, oracle, monkeypatch):
+    """Lists and frame vector above the limit: the tile kernel serves the call and no memory is taken.  Unsymmetric
+    integrals on one alpha electron, whose beta columns make the longest lists, within it."""
+    from binsim_b200 import cuotf, network as nw
+    sym = np.array([0, 1] * 7, np.int64)
+    net = _masked(14, sym, 0)
+    B = cuotf.CuBasis(14, 7, 7, orbsym=sym, num_irreps=2)
+    assert 8 * B.dim < 50e6 < 1.1 * 8 * B.dim   # the vector alone is just below the lowest limit, 0.05 GB
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+    x = cuda.randn(B.dim, dtype=cuda.float64, device="cuda")
+    y, z = cuda.empty_like(x), cuda.empty_like(x)
+    f.hvec_tiles(x, z, 0, f.num_tiles())
+    monkeypatch.setenv("BSIM_SIGMA_SCRATCH_GB", "0.05")
+    cuda.cuda.synchronize()
+    free = cuda.cuda.mem_get_info()[0]
+    f.hvec(x, y)
+    cuda.cuda.synchronize()
+    assert free - cuda.cuda.mem_get_info()[0] < 8e6
+    assert cuda.equal(y, z)
+    monkeypatch.delenv("BSIM_SIGMA_SCRATCH_GB")
+    sym = np.array([0, 1, 2, 3, 0, 1, 2, 3, 0], np.int64)
+    net = nw.hamiltonian_network(9, seed=1)
+    net.orbsym = sym
+    Bo = oracle.basis(9, 1, 4, orbsym=sym, num_irreps=4)
+    B = cuotf.CuBasis(9, 1, 4, orbsym=sym, num_irreps=4)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(net))
+    x = np.random.default_rng(9).normal(size=B.dim)
+    y = cuda.empty(B.dim, dtype=cuda.float64, device="cuda")
+    f.hvec(dev(cuda, x), y)
+    ref = oracle.hvec(Bo, oracle.network(net), x)
+    assert np.abs(y.cpu().numpy() - ref).max() <= 1e-13 * np.abs(ref).max()

@@ -1,5 +1,6 @@
 // Host-side construction of the structured sigma plan (see fastplan.h).
 #include "fastplan.h"
+#include "mixed.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -465,15 +466,25 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
             if (g >= 0) goff[(size_t)b * nFp + f] = (unsigned)(g >> 1) * 8u | (unsigned)(g & 1) << 31;
         }
     std::vector<int> lexp(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
-    for (int e = 0; e < P->nE; ++e) {
+    P->split = true;
+    for (int e = 0; e < P->nE && P->split; ++e) {
+        const double *row = &P->Lam[(size_t)e * P->nF];
         double m = 0.0;
-        bool bad = false;
         for (int f = 0; f < P->nF; ++f) {
-            const double v = std::fabs(P->Lam[(size_t)e * P->nF + f]);
-            bad = bad || !std::isfinite(v);
-            m = std::max(m, v);
+            if (!std::isfinite(row[f])) P->split = false;
+            m = std::max(m, std::fabs(row[f]));
         }
-        lexp[e] = bad ? 0x7fffffff : m > 0.0 ? std::ilogb(m) + 1 : -2000;
+        if (!P->split || m == 0.0) continue;
+        lexp[e] = std::ilogb(m) + 1;
+        int n = 0, far = 0;
+        for (int f = 0; f < P->nF; ++f) {
+            const double v = std::fabs(row[f]);
+            if (v == 0.0) continue;
+            ++n;
+            far += v < std::ldexp(1.0, lexp[e] - kFarBitsLam);
+            if (v < std::ldexp(1.0, lexp[e] - kLeastBits)) P->split = false;
+        }
+        if (8 * far > n) P->split = false;
     }
 
     // ---- intermediate-string tables ----------------------------------------------

@@ -112,6 +112,7 @@ struct FastPlan {
     const int *d_gidx = nullptr;       // [nF x ldG] (rank(b^F) << 1 | sign) or -1
     const unsigned *d_goff = nullptr;  // the same as byte offsets, by column (MixedArgs)
     const int *d_lexp = nullptr;       // [nE] exponent above a row of Lam
+    bool split = false;                // the rows of Lam suit the split products (sigma_split.cu)
     const int *d_resid = nullptr;      // residual group plan (for the generic kernel)
     const int4 *d_resid_chunks = nullptr;
     int n_resid_chunks = 0;

@@ -82,8 +82,11 @@ int mixed_tc_timeouts(int *count, bool reset);
 // The mixed product of the FP64 sigma as split products on the tensor cores
 // (sigma_split.cu), up to kSplitRows output rows per pass (from jbase).  It reads the
 // rows of c~ as fixed-point words with one exponent per row, which rows_to_fixed makes
-// in place.
+// in place.  A row whose elements spread too far for that keeps its FP64 elements and the
+// exponent kWideRow, and is left to mixed_dmma_kernel (the line: sigma_split.cu).
 constexpr int kSplitRows = 64;
+constexpr int kWideRow = 0x7fffffff;
+constexpr int kFarBits = 12, kFarBitsLam = 10, kLeastBits = 30;   // of elements: more than 1/8 below, one below
 // output rows per pass, 0: no kernel for the shape
 int mixed_split_rows(int nF, int M);
 int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s);

@@ -632,6 +632,7 @@ mixed_gemm_kernel(const MixedArgs P, const Ti *__restrict__ astr, const T *__res
 // synchronise inside the loop.  Lam_conn (the A fragments, read by every warp)
 // is staged once per CTA with rows g and g + 8 of each 16-row tile side by
 // side, so a lane's two A elements of a K step are one 16-byte load.
+// rexp (null: every row): the rows that the split products leave (kWideRow).
 constexpr int kDmmaLS = 34;   // double2 per F row: 32 + 2 (2 mod 8: conflict-free 16-byte fragment loads)
 inline size_t mixed_dmma_smem(int ldA, int nF, bool grow)
 {
@@ -641,7 +642,7 @@ inline size_t mixed_dmma_smem(int ldA, int nF, bool grow)
 template <typename Ti, bool GROW>
 __global__ void __launch_bounds__(512, 1)
 mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *__restrict__ ct,
-                  double *__restrict__ Z, int z0, int W, int jbase)
+                  double *__restrict__ Z, int z0, int W, int jbase, const int *__restrict__ rexp)
 {
     chain_wait();
     constexpr int NT = 512;
@@ -653,88 +654,94 @@ mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *
     int *conn = reinterpret_cast<int *>(lam + (size_t)Kp * kDmmaLS);        // [kMaxConn]
     int *sgn = conn + kMaxConn;                                              // [kMaxConn]
     __shared__ int wcnt[NT / 32], cnt;
-    const int a = blockIdx.x;
-    const int m = connected_excitations<NT>(P, (u64)astr[a], conn, sgn, wcnt, &cnt);
-    const int jm = min(64, m - jbase);   // output rows of this pass
-    if (jm <= 0) return;                 // uniform across the CTA
-    const double *grow = ct + (i64)a * P.ldA;
-    if (!GROW) {
-        const int4 *src = reinterpret_cast<const int4 *>(grow);
-        int4 *dst = reinterpret_cast<int4 *>(srow);
-        const int n16 = P.ldA / 2;
-        for (int i = threadIdx.x; i < n16; i += NT) dst[i] = __ldg(src + i);
-    }
-    // lam[f][8 rb + g] = (Lam_conn[16 rb + g][f], Lam_conn[16 rb + g + 8][f])
-    const double *Lam = static_cast<const double *>(P.Lam);
-    for (int i = threadIdx.x; i < Kp * kDmmaLS; i += NT) {
-        const int f = i / kDmmaLS, q = i % kDmmaLS;
-        const int j0 = (q >> 3) * 16 + (q & 7), j1 = j0 + 8;
-        double2 v = make_double2(0.0, 0.0);
-        if (q < 32 && f < K) {
-            if (j0 < jm) v.x = (double)sgn[jbase + j0] * Lam[(i64)conn[jbase + j0] * K + f];
-            if (j1 < jm) v.y = (double)sgn[jbase + j1] * Lam[(i64)conn[jbase + j1] * K + f];
+    for (int a = blockIdx.x; a < P.nA; a += gridDim.x) {
+        if (rexp && rexp[a] != kWideRow) continue;   // uniform: the split kernel computed this source row
+        const int m = connected_excitations<NT>(P, (u64)astr[a], conn, sgn, wcnt, &cnt);
+        const int jm = min(64, m - jbase);   // output rows of this pass
+        if (jm <= 0) {                       // uniform across the CTA
+            __syncthreads();
+            continue;
         }
-        lam[i] = v;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int nrb = (jm + 15) >> 4;   // 16-row tiles holding connected rows
-    const int zend = min(P.cend, z0 + W);
-    const int ncb = (zend - z0 + kMixCols - 1) / kMixCols;
-    const int nfc = (K + 31) / 32;
-    const int nsteps = ncb * nfc;
-    const int col = 8 * wid + g;     // this lane's B column within a chunk
-    int gp[8];
-    double gv[GROW ? 8 : 1];
-    auto load = [&](int step) {
-        const int cb = z0 + (step / nfc) * kMixCols, f0 = (step % nfc) * 32;
-        const int *gb = P.gidx + (i64)(f0 + t) * P.ldG + cb + col;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) gp[i] = f0 + 4 * i + t < K ? __ldg(gb + (i64)(4 * i) * P.ldG) : -1;
-        if constexpr (GROW) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) gv[i] = gp[i] >= 0 ? __ldg(grow + (gp[i] >> 1)) : 0.0;
+        const double *grow = ct + (i64)a * P.ldA;
+        if (!GROW) {
+            const int4 *src = reinterpret_cast<const int4 *>(grow);
+            int4 *dst = reinterpret_cast<int4 *>(srow);
+            const int n16 = P.ldA / 2;
+            for (int i = threadIdx.x; i < n16; i += NT) dst[i] = __ldg(src + i);
         }
-    };
-    double c[4][4];
-#pragma unroll
-    for (int rb = 0; rb < 4; ++rb) c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0;
-    if (nsteps > 0) load(0);
-    for (int step = 0; step < nsteps; ++step) {
-        const int cbi = step / nfc, fci = step % nfc;
-        const int f0 = fci * 32, nk = (min(32, K - f0) + 3) >> 2;
-        double x[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int gg = gp[i];
-            double v;
-            if constexpr (GROW) v = gv[i];
-            else v = gg >= 0 ? srow[gg >> 1] : 0.0;
-            x[i] = (gg >= 0 && (gg & 1)) ? -v : v;
+        // lam[f][8 rb + g] = (Lam_conn[16 rb + g][f], Lam_conn[16 rb + g + 8][f])
+        const double *Lam = static_cast<const double *>(P.Lam);
+        for (int i = threadIdx.x; i < Kp * kDmmaLS; i += NT) {
+            const int f = i / kDmmaLS, q = i % kDmmaLS;
+            const int j0 = (q >> 3) * 16 + (q & 7), j1 = j0 + 8;
+            double2 v = make_double2(0.0, 0.0);
+            if (q < 32 && f < K) {
+                if (j0 < jm) v.x = (double)sgn[jbase + j0] * Lam[(i64)conn[jbase + j0] * K + f];
+                if (j1 < jm) v.y = (double)sgn[jbase + j1] * Lam[(i64)conn[jbase + j1] * K + f];
+            }
+            lam[i] = v;
         }
-        if (step + 1 < nsteps) load(step + 1);
-        const double2 *la = lam + (size_t)(f0 + t) * kDmmaLS + g;
+        __syncthreads();
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+        const int nrb = (jm + 15) >> 4;   // 16-row tiles holding connected rows
+        const int zend = min(P.cend, z0 + W);
+        const int ncb = (zend - z0 + kMixCols - 1) / kMixCols;
+        const int nfc = (K + 31) / 32;
+        const int nsteps = ncb * nfc;
+        const int col = 8 * wid + g;     // this lane's B column within a chunk
+        int gp[8];
+        double gv[GROW ? 8 : 1];
+        auto load = [&](int step) {
+            const int cb = z0 + (step / nfc) * kMixCols, f0 = (step % nfc) * 32;
+            const int *gb = P.gidx + (i64)(f0 + t) * P.ldG + cb + col;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {   // K steps of 8: F rows f0 + 8i + t and f0 + 8i + 4 + t
-            if (2 * i < nk) {
+            for (int i = 0; i < 8; ++i) gp[i] = f0 + 4 * i + t < K ? __ldg(gb + (i64)(4 * i) * P.ldG) : -1;
+            if constexpr (GROW) {
 #pragma unroll
-                for (int rb = 0; rb < 4; ++rb)
-                    if (rb < nrb)
-                        dmma_16x8x8(c[rb], la[(size_t)(8 * i) * kDmmaLS + rb * 8],
-                                    la[(size_t)(8 * i + 4) * kDmmaLS + rb * 8], make_double2(x[2 * i], x[2 * i + 1]));
+                for (int i = 0; i < 8; ++i) gv[i] = gp[i] >= 0 ? __ldg(grow + (gp[i] >> 1)) : 0.0;
+            }
+        };
+        double c[4][4];
+#pragma unroll
+        for (int rb = 0; rb < 4; ++rb) c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0;
+        if (nsteps > 0) load(0);
+        for (int step = 0; step < nsteps; ++step) {
+            const int cbi = step / nfc, fci = step % nfc;
+            const int f0 = fci * 32, nk = (min(32, K - f0) + 3) >> 2;
+            double x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int gg = gp[i];
+                double v;
+                if constexpr (GROW) v = gv[i];
+                else v = gg >= 0 ? srow[gg >> 1] : 0.0;
+                x[i] = (gg >= 0 && (gg & 1)) ? -v : v;
+            }
+            if (step + 1 < nsteps) load(step + 1);
+            const double2 *la = lam + (size_t)(f0 + t) * kDmmaLS + g;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {   // K steps of 8: F rows f0 + 8i + t and f0 + 8i + 4 + t
+                if (2 * i < nk) {
+#pragma unroll
+                    for (int rb = 0; rb < 4; ++rb)
+                        if (rb < nrb)
+                            dmma_16x8x8(c[rb], la[(size_t)(8 * i) * kDmmaLS + rb * 8],
+                                        la[(size_t)(8 * i + 4) * kDmmaLS + rb * 8], make_double2(x[2 * i], x[2 * i + 1]));
+                }
+            }
+            if (fci == nfc - 1) {
+                double *zr = zchunk(Z, a, M, W, cbi) + (jbase + g) * kMixCols + 8 * wid + 2 * t;
+#pragma unroll
+                for (int rb = 0; rb < 4; ++rb) {
+                    if (rb < nrb && rb * 16 + g < jm)
+                        *reinterpret_cast<double2 *>(zr + rb * 16 * kMixCols) = make_double2(c[rb][0], c[rb][1]);
+                    if (rb < nrb && rb * 16 + g + 8 < jm)
+                        *reinterpret_cast<double2 *>(zr + (rb * 16 + 8) * kMixCols) = make_double2(c[rb][2], c[rb][3]);
+                    c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0;
+                }
             }
         }
-        if (fci == nfc - 1) {
-            double *zr = zchunk(Z, a, M, W, cbi) + (jbase + g) * kMixCols + 8 * wid + 2 * t;
-#pragma unroll
-            for (int rb = 0; rb < 4; ++rb) {
-                if (rb < nrb && rb * 16 + g < jm)
-                    *reinterpret_cast<double2 *>(zr + rb * 16 * kMixCols) = make_double2(c[rb][0], c[rb][1]);
-                if (rb < nrb && rb * 16 + g + 8 < jm)
-                    *reinterpret_cast<double2 *>(zr + (rb * 16 + 8) * kMixCols) = make_double2(c[rb][2], c[rb][3]);
-                c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0;
-            }
-        }
+        __syncthreads();   // the shared arrays are free for the next row
     }
 }
 
@@ -1267,7 +1274,7 @@ template <typename Ti>
 static int mixed_split(const FastPlan<Ti> &P)
 {
     const Split mode = split_mode();
-    if (mode == Split::never) return 0;
+    if (mode == Split::never || !P.split) return 0;
     if (mode == Split::automatic && (P.nB < kSplitMinCols || (double)P.nA * P.nB * P.nF < kSplitMinWork)) return 0;
     return mixed_split_rows(P.nF, P.M);
 }
@@ -1284,7 +1291,11 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                  sizeof(T) == 8 ? (const void *)P.d_Lam : (const void *)P.d_Lam32, P.d_gidx, P.d_goff, P.d_lexp};
     if constexpr (sizeof(T) == 8) {
         const int rows = mixed_split(P);
-        if (rows > 0) {   // split products; nothing reads c~ in floating point after this
+        const bool on_chip = mixed_dmma_smem(P.ldA, P.nF, false) <= std::min(kSmemMax, mixed_row_limit());
+        const size_t smem = mixed_dmma_smem(P.ldA, P.nF, !on_chip);
+        auto kern = on_chip ? mixed_dmma_kernel<Ti, false> : mixed_dmma_kernel<Ti, true>;
+        if (rows > 0 && smem <= kSmemMax) {   // split products; nothing reads a converted row in floating point after this
+            BSIM_CUDA(allow_smem(kern));
             int *rexp = reinterpret_cast<int *>(ct + (size_t)P.nA * P.ldA);   // behind the rows (run_fast)
             double *Z = static_cast<double *>(z.p);
             STAGE(tm, 0, s, rc = rows_to_fixed(ct, P.nA, P.ldA, rexp, s));
@@ -1294,6 +1305,9 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                     STAGE(tm, 3, s, rc = mixed_gemm_split<Ti>(ma, P.d_astr, ct, rexp, Z, z0, (int)z.w, jb, rows, s));
                     if (rc != BSIM_OK) return rc;
                 }
+                for (int jb = 0; jb < P.M; jb += 64)   // rows left in FP64: one CTA per SM looks for them
+                    STAGE(tm, 3, s, (launch_chained(kern, std::min(P.nA, 148), 512, smem, s, ma, P.d_astr, ct, Z, z0,
+                                                   (int)z.w, jb, (const int *)rexp)));
                 dim3 g(P.nA, (unsigned)((std::min<size_t>(z.w, c1 - z0) + kRowChunk - 1) / kRowChunk));
                 STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0,
                                                 (int)z.w)));
@@ -1346,7 +1360,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                 for (int z0 = c0; z0 < c1; z0 += (int)Wz) {
                     for (int pass = 0; pass < passes; ++pass)
                         STAGE(tm, 3, s, (launch_chained(kern, P.nA, 512, smem, s, ma, P.d_astr, ct, Z, z0, (int)Wz,
-                                                       64 * pass)));
+                                                       64 * pass, (const int *)nullptr)));
                     dim3 g(P.nA, (unsigned)((std::min<size_t>(Wz, c1 - z0) + kRowChunk - 1) / kRowChunk));
                     STAGE(tm, 4, s, (launch_chained(mixed_gather_kernel<Ti, T>, g, 256, 0, s, ma, B->view, Z, dst, z0, (int)Wz)));
                 }

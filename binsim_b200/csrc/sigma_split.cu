@@ -8,9 +8,19 @@
 // product and sum exact in 32-bit integers, the eight diagonals i + j = const summed in
 // 64 bits and rounded once (error-free splitting: Ozaki, Ogita, Oishi, Rump 2012; on
 // integer tensor cores: Ootomo, Ozaki, Yokota 2024).  The terms left out are below
-// 2^-59 of (largest element of the row) x (largest element of the B row); FP64 sums of
-// the same length round at 2^-53 of their terms.  Zeros stay exact.  A row whose
-// largest element is infinite or NaN gives NaN in its outputs.
+// 2^-57 of (largest element of the row) x (largest element of the B row) a product, and a
+// word's rounding below 2^-62 of its row's largest element.  FP64 rounds at 2^-53 of a
+// sum's own terms, so the split is as exact only where most elements of a row are not
+// far below its largest: a row of c~ with more than 1/8 of its nonzero elements below
+// 2^-12 of it (of the power of two above it), one below 2^-30 of it, or an infinity or
+// NaN, stays in FP64 and goes to mixed_dmma_kernel (kWideRow); a Hamiltonian with such a
+// row of Lam (1/8 below 2^-10) does not use the split products at all (fastplan.cu).
+// An output that only the few small elements of an accepted row reach keeps the bound
+// above, relative to the row.  Error over the sum of |terms| of an output, 36 terms, rms
+// and max of 4000, the byte products emulated on the host, FP64 / split: normal elements 5.3e-17 3.2e-16 / 1.2e-17 6.1e-17;
+// log-normal (sigma 1, 2 % below 2^-12) 7.2e-17 4.6e-16 / 2.4e-17 1.1e-16; log-uniform
+// over three decades (10 %) 9.0e-17 7.9e-16 / 2.6e-17 1.2e-16; beyond the line, log-normal
+// (sigma 2.5, 60 %) 1.2e-16 8.3e-16 / 3.3e-16 3.1e-15.  Zeros stay exact.
 //
 // The product is computed transposed, D[b][j], the 128 columns b of a chunk in
 // the MMA's M.  A byte plane i of X^T meets every byte plane j < 8 - i of B in
@@ -37,9 +47,9 @@
 // (bytes d + 128: a subtraction negates them) and byte offsets in the gather table.
 // Against mixed_dmma_kernel, which runs at the FP64 tensor rate: 0.426 -> 0.35 ms at
 // 12o 6+6, 1.05 -> 0.80 ms at 13o 7+5, 5.72 -> 3.83 ms at 14o 7+7, 99.8 -> 67.7 ms at
-// 16o 8+8, 1.29 -> 0.83 ms at 20o 3+3.  Errors of a sigma
-// against sums in extended precision, both kernels the same to 1 %: rms 2e-16, max 4e-16
-// of the largest output, on normal vectors and on ones over 6 and 12 decades.
+// 16o 8+8, 1.29 -> 0.83 ms at 20o 3+3.  On a vector whose rows all stay in FP64 (six
+// decades under a leading determinant, 13o 7+5) a sigma takes 2.16 ms, all rows split
+// 1.87.
 // Measured and not kept: FP16 digits (seven of 9 bits, kind::f16; 110 ms at 16o, for the
 // conversion of the digits), the same kernel for the doubles through intermediate
 // strings (43 -> 50 ms at 16o: 45 rows of 64, K of 45 in 64, coalesced DMMA operands)
@@ -49,7 +59,6 @@
 #include "tc.cuh"
 
 #include <algorithm>
-#include <climits>
 
 namespace bsim {
 
@@ -62,7 +71,6 @@ constexpr int kKS = 32;                    // K rows per slice: one MMA K step
 constexpr int kStages = 4;                 // A stages, at most
 constexpr int kRows = kSplitRows;          // output rows per pass
 constexpr uint32_t kPlane = kM * kKS;      // one byte plane of an A stage
-constexpr int kBadExp = INT_MAX;           // exponent of a row that holds an infinity or NaN
 constexpr int kZeroExp = -2000;            // exponent of a row of zeros
 
 // instruction descriptor of kind::i8: D S32 (bits 4-5 = 2), A and B signed (bits
@@ -138,13 +146,12 @@ __host__ __device__ inline SplitLayout split_layout(int K, int jm, uint32_t tab_
     L.total = o;
     return L;
 }
-constexpr int kRiRows = (kRiMaxU + kKS - 1) / kKS * kKS;
-constexpr uint32_t kMixTab = 2u * kMaxConn * 4u, kRiTab = (uint32_t)kRiRows * 12u;
+constexpr uint32_t kMixTab = 2u * kMaxConn * 4u;
 
 // smallest e with |x| < 2^e for the largest |x| = m of a row
 __device__ __forceinline__ int exp_above(double m)
 {
-    if (!(m <= 1.7976931348623157e308)) return kBadExp;   // infinite or NaN
+    if (!(m <= 1.7976931348623157e308)) return kWideRow;   // infinite or NaN
     return m > 0.0 ? ilogb(m) + 1 : kZeroExp;
 }
 // max that keeps a NaN
@@ -180,12 +187,14 @@ __device__ __forceinline__ void transpose4(uint32_t a, uint32_t b, uint32_t c, u
     out[3] = __byte_perm(z, w, 0x7632);
 }
 
-// Rows of c~ to fixed point in place, with the exponent of each.
+// Rows of c~ to fixed point in place, with the exponent of each; wide rows stay.
 __global__ void __launch_bounds__(256)
 rows_to_fixed_kernel(double *__restrict__ in, int ld, int *__restrict__ rexp)
 {
     chain_wait();
     __shared__ double red[8];
+    __shared__ int cnt[3];
+    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
     double *row = in + (i64)blockIdx.x * ld;
     double m = 0.0;
     for (int i = threadIdx.x; i < ld; i += 256) m = max_nan(m, fabs((double)row[i]));
@@ -194,10 +203,31 @@ rows_to_fixed_kernel(double *__restrict__ in, int ld, int *__restrict__ rexp)
     __syncthreads();
     m = red[0];
     for (int i = 1; i < 8; ++i) m = max_nan(m, red[i]);
-    const int e = exp_above(m);
-    if (threadIdx.x == 0) rexp[blockIdx.x] = e;
-    const bool plain = e != kBadExp && e != kZeroExp;
+    int e = exp_above(m);
+    const bool plain = e != kWideRow && e != kZeroExp;
     const Pow2 f(plain ? kBits - e : 0);
+    if (plain) {   // nonzero elements, those below 2^(e - kFarBits), those below 2^(e - kLeastBits)
+        const double far = ldexp(1.0, kBits - kFarBits), least = ldexp(1.0, kBits - kLeastBits);
+        int n = 0, k = 0, l = 0;
+        for (int i = threadIdx.x; i < ld; i += 256) {
+            const double x = fabs((double)row[i]), y = x * f.a * f.b;
+            n += x != 0.0;
+            k += x != 0.0 && y < far;
+            l += x != 0.0 && y < least;
+        }
+        n = __reduce_add_sync(0xffffffffu, n);
+        k = __reduce_add_sync(0xffffffffu, k);
+        l = __reduce_add_sync(0xffffffffu, l);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&cnt[0], n);
+            atomicAdd(&cnt[1], k);
+            atomicAdd(&cnt[2], l);
+        }
+        __syncthreads();
+        if ((i64)cnt[1] * 8 > cnt[0] || cnt[2] > 0) e = kWideRow;
+    }
+    if (threadIdx.x == 0) rexp[blockIdx.x] = e;
+    if (e == kWideRow) return;   // uniform across the CTA
     for (int i = threadIdx.x; i < ld; i += 256)
         reinterpret_cast<u64 *>(row)[i] = to_word(plain ? (double)row[i] : 0.0, f);
 }
@@ -205,7 +235,7 @@ rows_to_fixed_kernel(double *__restrict__ in, int ld, int *__restrict__ rexp)
 // B = [jm x K] as byte planes: row (half h, plane d, row e of the half) of one
 // K-major operand, and per output row the two factors whose product is
 // 2^(a_exp + its exponent - 68).  bval(j, k): the FP64 element, row_exp(j) the exponent
-// above row j.
+// above row j (kZeroExp for a row of zeros).
 template <typename BVal, typename RowExp>
 __device__ __forceinline__ void stage_b(const SplitLayout &L, unsigned char *smem, int jm, int K, int a_exp, BVal bval,
                                         RowExp row_exp)
@@ -213,15 +243,9 @@ __device__ __forceinline__ void stage_b(const SplitLayout &L, unsigned char *sme
     __shared__ double2 fj[kRows];
     if ((int)threadIdx.x < jm) {
         const int e = row_exp((int)threadIdx.x);
-        double2 f;
-        if (e == kBadExp || a_exp == kBadExp) f.x = f.y = __longlong_as_double(0x7ff8000000000000ll);
-        else {
-            const Pow2 p(a_exp + e - 2 * kBits + 8 * (ND - 1));
-            f = make_double2(p.a, p.b);
-        }
-        reinterpret_cast<double2 *>(smem + L.scale)[threadIdx.x] = f;
-        const Pow2 p(e == kBadExp || e == kZeroExp ? 0 : kBits - e);
-        fj[threadIdx.x] = e == kBadExp || e == kZeroExp ? make_double2(0.0, 0.0) : make_double2(p.a, p.b);
+        const Pow2 f(a_exp + e - 2 * kBits + 8 * (ND - 1)), p(e == kZeroExp ? 0 : kBits - e);
+        reinterpret_cast<double2 *>(smem + L.scale)[threadIdx.x] = make_double2(f.a, f.b);
+        fj[threadIdx.x] = e == kZeroExp ? make_double2(0.0, 0.0) : make_double2(p.a, p.b);
     }
     __syncthreads();
     const int n0 = half_rows(jm, 0), n1 = half_rows(jm, 1), nk4 = L.kp / 4;
@@ -558,6 +582,7 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, const u6
     __shared__ volatile int abort_flag;
     __shared__ int skip_all;
     const int a = blockIdx.x;
+    if (rexp[a] == kWideRow) return;   // uniform across the CTA: mixed_dmma_kernel computes the row
     if (threadIdx.x == 0) skip_all = *(volatile int *)&g_tc_abort;
     __syncthreads();
     if (skip_all) return;   // an earlier CTA gave up a wait: the result is void (counted)

@@ -153,7 +153,14 @@ int bsim_network_from_host(void *host_net, void **out);
 int bsim_network_destroy(void *net);
 int64_t bsim_network_ngs(void *net);
 
-/* dst = H src, FP64. */
+/* dst = H src, FP64.  On single-block bases above a size line the mixed
+ * single-single excitations go through fixed-point words of 62 bits below the
+ * largest element of an alpha row of src, multiplied exactly.  A row keeps FP64
+ * elements and sums when more than 1/8 of its nonzero elements lie below 2^-12
+ * of that largest one, any below 2^-30 of it, or it holds an infinity or NaN.
+ * So the error of an output is that of FP64 sums of its own terms, except for an
+ * output that only the few small elements of a row reach: there it is up to
+ * 2^-57 of (the row's largest element) x (the largest integral) a term. */
 int bsim_hvec(void *basis, void *net, const double *src, double *dst, bsim_stream_t stream);
 /* sigma of nvec HOST vectors: dst_host[k] = H src_host[k] (dim doubles each;
  * the same host buffer may appear in several slots).  The library holds two

@@ -89,10 +89,11 @@ constexpr int kWideRow = 0x7fffffff;
 constexpr int kFarBits = 12, kFarBitsLam = 10, kLeastBits = 30;   // of elements: more than 1/8 below, one below
 // output rows per pass, 0: no kernel for the shape
 int mixed_split_rows(int nF, int M);
+// rexp: [rows] exponents and the call's flag of waits that gave up
 int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s);
 template <typename Ti>
-int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, const double *ct, const int *rexp, double *Z, int z0, int W,
-                     int jbase, int rows, cudaStream_t s);
+int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, double *ct, int *rexp, double *Z, int z0, int W, int jbase,
+                     int rows, cudaStream_t s);
 int split_timeouts(int *count, bool reset);
 
 }  // namespace bsim

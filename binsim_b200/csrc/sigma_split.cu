@@ -36,7 +36,9 @@
 //               slices ahead in registers, and write their bytes as K-major core
 //               matrices, one (column, 8 rows) group per thread;
 //   warp 24     TMEM allocation and, by one lane, the MMA issue.
-// Handoffs and bounded waits as in sigma_tc.cu.
+// Handoffs and bounded waits as in sigma_tc.cu; a CTA that gives up a wait, and every
+// CTA of the call that starts after it, leaves its row to mixed_dmma_kernel
+// (row_to_fp64).
 //
 // Bound: the L1 pipe that the producers' gathers, the byte stores and the epilogue's
 // stores share (a slice of 4 K words takes ~3700 cycles, the MMAs of 64 rows 1200 of
@@ -59,6 +61,7 @@
 #include "tc.cuh"
 
 #include <algorithm>
+#include <cstdlib>
 
 namespace bsim {
 
@@ -227,6 +230,7 @@ rows_to_fixed_kernel(double *__restrict__ in, int ld, int *__restrict__ rexp)
         if ((i64)cnt[1] * 8 > cnt[0] || cnt[2] > 0) e = kWideRow;
     }
     if (threadIdx.x == 0) rexp[blockIdx.x] = e;
+    if (blockIdx.x == 0 && threadIdx.x == 0) rexp[gridDim.x] = 0;   // the call's flag of waits that gave up
     if (e == kWideRow) return;   // uniform across the CTA
     for (int i = threadIdx.x; i < ld; i += 256)
         reinterpret_cast<u64 *>(row)[i] = to_word(plain ? (double)row[i] : 0.0, f);
@@ -377,23 +381,29 @@ __device__ __forceinline__ double sum4(int a, int b, int c, int d)
 {
     return unmagic(mad_wide(d, 1, mad_wide(c, 256, mad_wide(b, 65536, mad_wide(a, 16777216, kMagic)))));
 }
-// mbar_wait by every lane of a warp, with one answer for all
-__device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, volatile int *abort_flag)
+// A CTA's flag and the call's flag of waits that gave up (tc.cuh).
+struct GaveUp {
+    volatile int *cta;
+    int *call;
+};
+// mbar_wait by every lane of a warp, with one answer for all: what follows it is a
+// barrier of the warp or an aligned instruction
+__device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, const GaveUp &gu)
 {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, gu.cta, gu.call));
 }
 
 // The producers' loop: slice q into A stage q % kStages.
 template <typename Src>
 __device__ __forceinline__ void produce_slices(const SplitLayout &L, unsigned char *smem, uint32_t bar0, int nq, Src &src,
-                                               volatile int *abort_flag)
+                                               const GaveUp &gu)
 {
     const ProdPlace P((int)(threadIdx.x >> 5) - kEpiWarps, (int)(threadIdx.x & 31));
     src.begin(P);
     int st = 0;
     uint32_t empty = 1;   // parity before the first release: passes at once
     auto one = [&](auto set, int q) {
-        if (!mbar_wait(bar0 + 8u * (uint32_t)(kStages + st), empty, abort_flag)) return false;
+        if (!wait_all(bar0 + 8u * (uint32_t)(kStages + st), empty, gu)) return false;
         src.template put<decltype(set)::value>(q, P, smem + L.a + (size_t)st * kStageBytes);
         fence_async_smem();
         warp_arrive(bar0 + 8u * (uint32_t)st);
@@ -429,7 +439,7 @@ __device__ __forceinline__ void issue_planes(const SplitLayout &L, uint32_t sbas
 template <typename Src>
 __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned char *smem, uint32_t sbase, uint32_t tmem,
                                             int ncb, int jm, double *zrow, int zrows, Src &src,
-                                            volatile int *abort_flag)
+                                            const GaveUp &gu, bool drop)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bar0 = sbase + L.bars;   // afull[S], aempty[S], dfull[2], dempty[2], done
@@ -442,7 +452,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
     const int n0 = half_rows(jm, 0), n1 = half_rows(jm, 1), nh = n1 ? 2 : 1, nu = ncb * nh;
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kProdWarps) {
-        produce_slices(L, smem, bar0, ncb * nsl, src, abort_flag);
+        if (!drop) produce_slices(L, smem, bar0, ncb * nsl, src, gu);
     } else if (warp == kMmaWarp) {
         // ---- MMA issue (one elected lane).  With a chunk's slices all in stages, half by
         // half, so that one half's accumulator is read out during the other's MMAs; else
@@ -463,13 +473,13 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
                     st = st0;
                     full = full0;
                     // the accumulator's previous part was read out
-                    if (so == 0 && u >= 2 && !wait_all(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), abort_flag)) {
+                    if (so == 0 && u >= 2 && !wait_all(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), gu)) {
                         ok = false;
                         break;
                     }
                     for (int si = 0; si < nin; ++si) {
                         const int s = so * nin + si;
-                        if (h == 0 && !wait_all(afull(st), full, abort_flag)) { ok = false; break; }
+                        if (h == 0 && !wait_all(afull(st), full, gu)) { ok = false; break; }
                         tc_fence_after();
                         if (lead) {
                             issue_planes(L, sbase, st, s, boff, n, tmem + (uint32_t)(ND * n0 * acc));
@@ -485,7 +495,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
             }
         if (lead) umma_commit(done);   // every issued MMA has completed before TMEM is freed
         __syncwarp();
-        if (lane == 0) mbar_wait_drain(done, 0u);
+        if (lane == 0) mbar_wait_drain(done, 0u, gu.call);
         __syncwarp();
     } else if (warp < kEpiWarps) {
         // ---- epilogue: half of the part's rows per warp, eight at a time ----
@@ -493,7 +503,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
         const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         for (int u = 0; u < nu; ++u) {
             const int c = u / nh, h = u % nh, acc = u & 1;
-            if (!mbar_wait(dfull(acc), (uint32_t)((u >> 1) & 1), abort_flag)) break;
+            if (!wait_all(dfull(acc), (uint32_t)((u >> 1) & 1), gu)) break;
             tc_fence_after();
             const int n = h ? n1 : n0, e0 = (warp >> 2) * (n / 2), e1 = min(e0 + n / 2, jm - kHalf * h);
             const uint32_t base = lanes + (uint32_t)(ND * n0 * acc);
@@ -565,10 +575,21 @@ __device__ __forceinline__ void split_end(uint32_t tmem, uint32_t cols)
 // tensor memory of a pass: two accumulators of ND n columns, a power of two
 __device__ __forceinline__ uint32_t split_cols(int cols) { return cols > 256 ? 512u : cols > 128 ? 256u : 128u; }
 
+// A row's words back to FP64, and the row to mixed_dmma_kernel: the end of a CTA whose
+// waits gave up, so that a stalled device costs time and never a result.  The elements
+// are those of the words, within 2^-63 of the row's largest.
+__device__ void row_to_fp64(u64 *row, int ld, int e, int *rexp)
+{
+    const Pow2 f(e - kBits);
+    for (int i = threadIdx.x; i < ld; i += kThreads)
+        reinterpret_cast<double *>(row)[i] = (double)(long long)(row[i] - kBias) * f.a * f.b;
+    if (threadIdx.x == 0) *rexp = kWideRow;
+}
+
 template <typename Ti>
 __global__ void __launch_bounds__(kThreads, 1)
-mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, const u64 *__restrict__ ct,
-                     const int *__restrict__ rexp, double *__restrict__ Z, int z0, int W, int jbase, int rows)
+mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, u64 *ct, int *rexp, double *__restrict__ Z,
+                        int z0, int W, int jbase, int rows, int drop)
 {
     chain_wait();
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -581,17 +602,22 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, const u6
     __shared__ int wcnt[kThreads / 32], cnt;
     __shared__ volatile int abort_flag;
     __shared__ int skip_all;
-    const int a = blockIdx.x;
-    if (rexp[a] == kWideRow) return;   // uniform across the CTA: mixed_dmma_kernel computes the row
-    if (threadIdx.x == 0) skip_all = *(volatile int *)&g_tc_abort;
+    const int a = blockIdx.x, aexp = rexp[a];
+    int *call_flag = rexp + P.nA;
+    u64 *row = ct + (i64)a * P.ldA;
+    if (aexp == kWideRow) return;   // uniform across the CTA: mixed_dmma_kernel computes the row
+    if (threadIdx.x == 0) skip_all = *(volatile int *)call_flag;
     __syncthreads();
-    if (skip_all) return;   // an earlier CTA gave up a wait: the result is void (counted)
+    if (skip_all) {   // an earlier CTA gave up a wait
+        row_to_fp64(row, P.ldA, aexp, rexp + a);
+        return;
+    }
     const int m = connected_excitations<kThreads>(P, (u64)astr[a], conn, sgn, wcnt, &cnt);
     const int jm = min(jcap, m - jbase);
     if (jm <= 0) return;   // uniform across the CTA
     const double *Lam = static_cast<const double *>(P.Lam);
     stage_b(
-        L, smem, jm, K, rexp[a],
+        L, smem, jm, K, aexp,
         [&](int j, int f) { return (double)sgn[jbase + j] * __ldg(Lam + (i64)conn[jbase + j] * K + f); },
         [&](int j) { return __ldg(P.lexp + conn[jbase + j]); });
     const uint32_t cols = split_cols(2 * ND * half_rows(jm, 0));
@@ -600,14 +626,16 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, const u6
     const int ncb = (zend - z0 + kM - 1) / kM;
     GatherWords src;
     src.goff = P.goff;
-    src.row = reinterpret_cast<const unsigned char *>(ct + (i64)a * P.ldA);
+    src.row = reinterpret_cast<const unsigned char *>(row);
     src.ldG = P.ldG;
     src.kp = L.kp;
     src.z0 = z0;
     src.nsl = L.kp / kKS;
     src.nq = ncb * src.nsl;
-    split_pipeline(L, smem, sbase, tmem, ncb, jm, zchunk(Z, a, P.M, W, 0) + jbase * kM, P.M, src, &abort_flag);
+    split_pipeline(L, smem, sbase, tmem, ncb, jm, zchunk(Z, a, P.M, W, 0) + jbase * kM, P.M, src,
+                   GaveUp{&abort_flag, call_flag}, a == drop);
     split_end(tmem, cols);
+    if (abort_flag) row_to_fp64(row, P.ldA, aexp, rexp + a);   // uniform: written before split_end's barrier
 }
 
 }  // namespace
@@ -618,7 +646,6 @@ int mixed_split_rows(int nF, int M)
         if (split_layout(nF, std::min(M, rows), kMixTab).total + kStaticSmem <= kSmemMax) return rows;
     return 0;
 }
-static const u64 *words(const double *p) { return reinterpret_cast<const u64 *>(p); }
 
 int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s)
 {
@@ -629,13 +656,17 @@ int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s)
 }
 
 template <typename Ti>
-int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, const double *ct, const int *rexp, double *Z, int z0, int W,
-                     int jbase, int rows, cudaStream_t s)
+int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, double *ct, int *rexp, double *Z, int z0, int W, int jbase,
+                     int rows, cudaStream_t s)
 {
+    // BSIM_SPLIT_DROP_ROW (tests): the producers of this row fill nothing, so the row's
+    // waits run out
+    const char *drop = getenv("BSIM_SPLIT_DROP_ROW");
     const size_t smem = split_layout(ma.nF, std::min(rows, ma.M - jbase), kMixTab).total;
     auto kern = mixed_gemm_split_kernel<Ti>;
     BSIM_CUDA(allow_smem(kern));
-    launch_chained(kern, ma.nA, kThreads, smem, s, ma, astr, words(ct), rexp, Z, z0, W, jbase, rows);
+    launch_chained(kern, ma.nA, kThreads, smem, s, ma, astr, reinterpret_cast<u64 *>(ct), rexp, Z, z0, W, jbase, rows,
+                   drop ? atoi(drop) : -1);
     BSIM_CUDA(cudaGetLastError());
     return BSIM_OK;
 }
@@ -647,15 +678,14 @@ int split_timeouts(int *count, bool reset)
     if (reset) {
         const int z = 0;
         BSIM_CUDA(cudaMemcpyToSymbol(g_tc_timeouts, &z, sizeof(int)));
-        BSIM_CUDA(cudaMemcpyToSymbol(g_tc_abort, &z, sizeof(int)));
     }
     *count = h;
     return BSIM_OK;
 }
 
-template int mixed_gemm_split<unsigned>(const MixedArgs &, const unsigned *, const double *, const int *, double *, int,
-                                        int, int, int, cudaStream_t);
-template int mixed_gemm_split<unsigned long long>(const MixedArgs &, const unsigned long long *, const double *,
-                                                  const int *, double *, int, int, int, int, cudaStream_t);
+template int mixed_gemm_split<unsigned>(const MixedArgs &, const unsigned *, double *, int *, double *, int, int, int,
+                                        int, cudaStream_t);
+template int mixed_gemm_split<unsigned long long>(const MixedArgs &, const unsigned long long *, double *, int *, double *,
+                                                  int, int, int, int, cudaStream_t);
 
 }  // namespace bsim

@@ -112,9 +112,11 @@ int64_t bsim_device_alloc_count(void);
  * out of memory. */
 int bsim_release_cached_memory(void);
 /* No counterpart in the reference.  Waits inside the library's tensor-core
- * (tcgen05) kernels are bounded; a wait that gives up makes its CTA skip the
- * rest of its work (the result is then wrong) and is counted.  *count = the
- * count on the current device since the last reset (0 in normal operation);
+ * (tcgen05) kernels are bounded; a wait that gives up is counted.  In the FP64
+ * sigma the CTA's row is then computed by another kernel: the call takes longer
+ * and its result is good.  In the FP32-bulk sigma the CTA, and every later one
+ * until the reset, skips the rest of its work: the result is wrong.  *count =
+ * the count on the current device since the last reset (0 in normal operation);
  * reset != 0 clears it.  Synchronous (reads device memory). */
 int bsim_tensor_core_timeouts(int32_t *count, int32_t reset);
 

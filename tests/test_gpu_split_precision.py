@@ -92,3 +92,31 @@ def test_non_finite_elements_reach_what_they_reached(cuda, system, monkeypatch):
         assert bool(cuda.isfinite(z).any())
         assert cuda.equal(cuda.isfinite(y), cuda.isfinite(z))
         assert cuda.equal(cuda.isnan(y), cuda.isnan(z))
+
+
+def test_a_wait_that_runs_out_costs_no_result(cuda, system, monkeypatch):
+    """The producers of one row fill nothing: its waits run out (20 ms, counted), the row and those after it go to the FP64
+    kernel, and the next call is as before."""
+    import ctypes as C
+    from binsim_b200.cuotf import lib
+    B, f, _ = system
+    x = dev(cuda, _vector("normal", B.dim))
+    y, z, w = (cuda.full_like(x, float("nan")) for _ in range(3))
+
+    def timeouts(reset):
+        n = C.c_int32()
+        assert lib().bsim_tensor_core_timeouts(C.byref(n), reset) == 0
+        return n.value
+    timeouts(1)
+    monkeypatch.setenv("BSIM_SIGMA_SPLIT", "1")
+    f.hvec(x, z)
+    for row in (0, 33, 69):
+        monkeypatch.setenv("BSIM_SPLIT_DROP_ROW", str(row))
+        f.hvec(x, y)
+        # the row's elements are its words, within 2^-63 of its largest; both kernels as in the test above
+        assert float((y - z).abs().max()) <= 1e-13 * float(z.abs().max())
+        assert timeouts(1) >= 1
+    monkeypatch.delenv("BSIM_SPLIT_DROP_ROW")
+    f.hvec(x, w)
+    assert cuda.equal(w, z)
+    assert timeouts(0) == 0

@@ -304,7 +304,8 @@ __device__ __forceinline__ void tc_pipeline(const TcLayout &L, unsigned char *sm
         // ---- epilogue: D (TMEM lanes 32 warp .. +31 = columns b) -> Z[row][j][b] ----
         for (int c = 0; c < ncb; ++c) {
             const int dbuf = c & 1;
-            if (!mbar_wait(dfull(dbuf), (uint32_t)((c >> 1) & 1), abort_flag, &g_tc_abort)) break;
+            // one answer for the warp: the tensor-memory loads below are aligned
+            if (!__all_sync(0xffffffffu, mbar_wait(dfull(dbuf), (uint32_t)((c >> 1) & 1), abort_flag, &g_tc_abort))) break;
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)dbuf * N;
             float *zb = zrow + (i64)c * zrows * kTcM + warp * 32 + lane;

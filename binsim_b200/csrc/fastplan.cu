@@ -457,15 +457,8 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
             }
     }
 
-    // the same as byte offsets into rows of 8-byte words, by column, F to whole slices
-    const int nFp = (P->nF + 31) & ~31;
-    std::vector<unsigned> goff((size_t)P->ldG * nFp, (unsigned)nB * 8u);
-    for (int f = 0; f < P->nF; ++f)
-        for (int b = 0; b < nB; ++b) {
-            const int g = gidx[(size_t)f * P->ldG + b];
-            if (g >= 0) goff[(size_t)b * nFp + f] = (unsigned)(g >> 1) * 8u | (unsigned)(g & 1) << 31;
-        }
-    std::vector<int> lexp(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
+    std::vector<int> &lexp = P->lexp;
+    lexp.assign(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
     P->split = true;
     for (int e = 0; e < P->nE && P->split; ++e) {
         const double *row = &P->Lam[(size_t)e * P->nF];
@@ -559,7 +552,6 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     auto bytes = [](size_t n, size_t sz) { return ((std::max<size_t>(n, 1) * sz) + 255) & ~size_t(255); };
     size_t tot = bytes(nA, sizeof(Ti)) + bytes(nB, sizeof(Ti)) + bytes(nA, 8) + bytes(PAd.size(), 8) +
                  bytes(PBd.size(), 8) + 2 * bytes(P->nE, 8) + 2 * bytes(P->Lam.size(), 8) + bytes(gidx.size(), 4) +
-                 bytes(goff.size(), 4) + bytes(lexp.size(), 4) +
                  bytes(P->residual.size(), 4) + bytes(P->residual.size() + 1, 16);
     for (int li = 0; li < 3; ++li)
         tot += 2 * bytes(csr[li].cptr.size(), 8) + bytes(csr[li].cent.size(), sizeof(CEnt)) +
@@ -587,8 +579,6 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     std::vector<float> lam32(P->Lam.begin(), P->Lam.end());
     P->d_Lam32 = put(lam32);
     P->d_gidx = put(gidx);
-    P->d_goff = put(goff);
-    P->d_lexp = put(lexp);
     for (int li = 0; li < 3; ++li) {
         CSRHost &C = csr[li];
         if (li == 2 && !ri_on[1]) continue;

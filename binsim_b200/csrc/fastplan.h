@@ -110,8 +110,7 @@ struct FastPlan {
     const float *d_Lam32 = nullptr;
     const double *d_PBdT = nullptr;    // [rank_d x ldA] beta diagonal factors, transposed
     const int *d_gidx = nullptr;       // [nF x ldG] (rank(b^F) << 1 | sign) or -1
-    const unsigned *d_goff = nullptr;  // the same as byte offsets, by column (MixedArgs)
-    const int *d_lexp = nullptr;       // [nE] exponent above a row of Lam
+    std::vector<int> lexp;             // [nE] exponent above a row of Lam
     bool split = false;                // the rows of Lam suit the split products (sigma_split.cu)
     const int *d_resid = nullptr;      // residual group plan (for the generic kernel)
     const int4 *d_resid_chunks = nullptr;

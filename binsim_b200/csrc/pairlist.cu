@@ -70,14 +70,22 @@ int build_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> *P)
     bmap.reserve((size_t)nB * 2);
     for (int a = 0; a < nA; ++a) amap[(u64)B->astrs[a]] = a;
     for (int b = 0; b < nB; ++b) bmap[(u64)B->bstrs[b]] = b;
-    std::vector<int2> alist, blist;
+    std::vector<int2> alist, blist, lower;
     std::unordered_map<u64, int2> aidx, bidx;   // mask -> {offset, count} (beta: count of the whole list)
     std::unordered_map<u64, int> bhalf;         // beta mask -> entries with partner index above
+    // flipping x keeps the electron count, and so may lead to a string of the basis, only
+    // where the string holds half of x's orbitals (bits are counted by clearing them: few).
+    // The first gradient of the 20o 3a3b pool: 229 -> 72 ms
+    auto half = [](u64 s, int n) {
+        for (; s && n > 0; s &= s - 1) --n;
+        return n == 0 && s == 0;
+    };
     auto alpha_list = [&](u64 x) {
         auto it = aidx.find(x);
         if (it != aidx.end()) return it->second;
-        const int off = (int)alist.size();
+        const int off = (int)alist.size(), nx = __builtin_popcountll(x), n2 = (nx & 1) ? -1 : nx / 2;
         for (int a = 0; a < nA; ++a) {
+            if (!half((u64)B->astrs[a] & x, n2)) continue;
             auto f = amap.find((u64)B->astrs[a] ^ x);
             if (f != amap.end() && f->second > a) alist.push_back(make_int2(a, f->second));
         }
@@ -88,16 +96,17 @@ int build_pair_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, PairPlan<Ti> *P)
     auto beta_list = [&](u64 x) {
         auto it = bidx.find(x);
         if (it != bidx.end()) return it->second;
-        const int off = (int)blist.size();
+        const int off = (int)blist.size(), nx = __builtin_popcountll(x), n2 = (nx & 1) ? -1 : nx / 2;
+        lower.clear();
         for (int b = 0; b < nB; ++b) {   // partner index above first: the pure-beta half
+            if (!half((u64)B->bstrs[b] & x, n2)) continue;
             auto f = bmap.find((u64)B->bstrs[b] ^ x);
-            if (f != bmap.end() && f->second > b) blist.push_back(make_int2(b, f->second));
+            if (f == bmap.end()) continue;
+            if (f->second > b) blist.push_back(make_int2(b, f->second));
+            if (f->second < b) lower.push_back(make_int2(b, f->second));
         }
         bhalf[x] = (int)blist.size() - off;
-        for (int b = 0; b < nB; ++b) {
-            auto f = bmap.find((u64)B->bstrs[b] ^ x);
-            if (f != bmap.end() && f->second < b) blist.push_back(make_int2(b, f->second));
-        }
+        blist.insert(blist.end(), lower.begin(), lower.end());
         const int2 r = make_int2(off, (int)blist.size() - off);
         bidx[x] = r;
         return r;

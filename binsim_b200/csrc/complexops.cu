@@ -292,7 +292,10 @@ int c64_build(const DevBasis<Ti> *B, const DevNet<Ti> *N, C64Lists *P, cudaStrea
     }
     for (size_t i = 0; i < row.size(); ++i) start[i + 1] = start[i] + count[i];
     int st = BSIM_OK;
-    const bool fits = tables + (double)start.back() * sizeof(C64Ent) <= (double)kC64Tables;
+    // at most half of the free memory, too: the plans of every live basis stay
+    size_t free_b = 0, total_b = 0;
+    if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &total_b);
+    const bool fits = tables + (double)start.back() * sizeof(C64Ent) <= std::min((double)kC64Tables, 0.5 * (double)free_b);
     if (e == cudaSuccess && fits) {
         st = P->arena.reserve(al(row.size() * 8) + al(start.size() * 8) + al((size_t)start.back() * sizeof(C64Ent) + 1) +
                               al(masks.size() * P->nBt * 4) + al((size_t)rows * P->nBt * sizeof(cx) + 1));

@@ -32,7 +32,7 @@ namespace bsim {
 
 constexpr int kRowChunk = 1024;        // columns per CTA in the gather kernels (256 threads x 4)
 template <typename T> constexpr int kRowThreads = sizeof(T) == 8 ? 256 : 384;   // of a CTA of pure_rows_kernel
-constexpr int kSplitCtas = 512;        // below this many CTAs of the row kernel: pure_split_kernel (measured there)
+constexpr int kSplitCtas = 512;        // below this many CTAs of the row kernel: pure_split_kernel (both sides there)
 
 template <typename T> struct Vec2;
 template <> struct Vec2<double> { using type = double2; };
@@ -193,9 +193,12 @@ pure_rows_kernel(int row_begin, int col_begin, int ncols, int ld_in, const SideC
 // to warp e % 8, the warps' sums added in order), 128 columns per CTA: for sizes
 // that leave pure_rows_kernel a few CTAs per SM, each walking its entries one
 // dependent load after another.  Alpha + beta rows, us, FP64, by the CTAs of the
-// other kernel: 38.4 -> 17.3 at 8o (70), 51.9 -> 27.6 at 10o (252), 62.9 -> 55.6 at
-// 11o 5+5 (462); 154.7 -> 150.3 at 12o 5+5 (792); 172.5 -> 192.9 at 12o 6+6 (924),
-// where the column tables read by every CTA of a row cost more than the waits.
+// other kernel: 38.3 -> 17.0 at 8o 4+4 (70), 52.4 -> 27.4 at 10o 5+5 (252), 64.7 -> 56.4
+// at 11o 5+5 (462), 74.5 -> 61.2 at 12o 4+4 (495); 95.2 -> 117.5 at 13o 4+4 (715), 170.7 ->
+// 191.1 at 12o 6+6 (924), 280.3 -> 387.8 at 13o 5+5 (2574), where the column tables read
+// by every CTA of a row cost more than the waits.  Between the last gain and the first
+// loss on both sides lies kSplitCtas.  Long lists of entries move the line up: 153.0 ->
+// 146.5 at 12o 5+5 (792), 208 -> 185 at 16o 3+3 (560), 552 -> 429 at 18o 3+3 (816).
 constexpr int kSplitCols = 128;
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -1262,15 +1265,18 @@ static Split split_mode()
 }
 
 // Output rows per pass of the split mixed product, 0: the DMMA kernels.  The split
-// kernel works on chunks of 128 columns and needs two to keep its warps busy, and its
-// rows_to_fixed and staging cost ~8 us (both kernels, us, DMMA / split): one chunk
-// loses, 312 / 353 at 14o 7+2 (91 columns), 908 / 1039 at 16o 6+2 (120); so do small
-// products, 12.4 / 21.1 at 10o 3+3, 29.7 / 35.4 at 10o 5+5 (2.9 M rows x columns x F);
-// 41.2 / 39.4 at 12o 3+3 (3.2 M), 72 / 48 at 18o 2+2 (3.6 M, 153 columns), 101 / 85 at
-// 11o 5+5 (11.7 M), 1295 / 837 at 20o 3+3.  By the whole basis, not by the call's
-// columns: column bands of one sigma give the same bits however they are cut.
+// kernel works on chunks of 128 columns and needs two to keep its warps busy: one chunk
+// loses, DMMA / split 312 / 353 us at 14o 7+2 (91 columns), 908 / 1039 at 16o 6+2 (120).
+// rows_to_fixed, the staging and the launch for rows left in FP64 cost ~12 us, which
+// small products (rows x columns x F) do not earn back.  A whole sigma, us, DMMA / split:
+// 73.3 / 78.5 at 10o 4+4 (2.0 M), 86.3 / 91.3 at 10o 5+5 (2.9 M), 101.4 / 101.9 at 12o 3+3
+// (3.2 M); 107.0 / 84.9 at 18o 2+2 (3.6 M, K of 153), 143.0 / 141.0 at 11o 4+4 (6.0 M),
+// 231.6 / 220.3 at 11o 5+5 (11.7 M), 263.6 / 233.3 at 12o 4+4 (16 M).  The gain grows with
+// K too, but no size between the last loss and the first gain was seen to be far off.  By
+// the whole basis, not by the call's columns: column bands of one sigma give the same
+// bits however they are cut.
 constexpr int kSplitMinCols = 129;
-constexpr double kSplitMinWork = 3.1e6;
+constexpr double kSplitMinWork = 3.4e6;
 template <typename Ti>
 static int mixed_split(const FastPlan<Ti> &P)
 {

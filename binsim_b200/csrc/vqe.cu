@@ -95,7 +95,9 @@ int vqe_energy_grad(const DevBasis<Ti> *B, const DevNet<Ti> *H, const DevNet<Ti>
             if ((i == 0 || param_idx[i] != param_idx[i - 1]) && param_idx[i] % ckpt_every == 0 && i > 0)
                 ck_pos.push_back(i);
     // checkpoints, gradient terms, scalars and the reduction scratch live in the
-    // basis workspace (grown on demand, kept between calls): no allocation per call
+    // basis workspace (grown on demand, kept between calls).  The orbit lists of the
+    // units and their partial sums come from the library's pool, which keeps them for
+    // the next call; making them waits for the stream once (RotSequence::init)
     const size_t n_ck = (size_t)n * ck_pos.size(), n_terms = (size_t)std::max<i64>(1, n_ops);
     void *wsp = nullptr;
     TRY(workspace_for(B).general(sizeof(double) * (n_ck + n_terms + 8 + kDavPartDoubles + kDavResDoubles), &wsp));

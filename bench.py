@@ -275,7 +275,7 @@ def profile_traffic(name):
         return None
 
 
-def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma_peak=None):
+def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms):
     """Roofline of the dominant kernel of the structured sigma, from the per-stage
     CUDA-event times measured in this run.  Returns (roofline dict, launches per sigma)."""
     if not stages:
@@ -290,7 +290,7 @@ def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma
         kern[name] = (t0 + t, n0 + n)
     top = max(kern, key=lambda k: kern[k][0])
     t_ms, n_launch = kern[top]
-    per_launch_s = t_ms * 1e-3 / max(1, n_launch)
+    stage_s = t_ms * 1e-3   # of one sigma, all launches of the stage
     nA, nB = math.comb(cfg["norb"], cfg["na"]), math.comb(cfg["norb"], cfg["nb"])
     types = net.type_codes()
     if top == "mixed_gemm":
@@ -299,9 +299,6 @@ def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma
         M = cfg["na"] * (cfg["norb"] - cfg["na"])
         bytes_total = dim * 8.0 + nA * M * nB * 8.0
         flops_total = float(np.sum(pairs[types == 3] * (2 * net.ranks[types == 3] + 1)))
-        # the GEMMs as executed: 64-row passes x every F excitation x every column
-        nF = math.comb(cfg["norb"], 2)
-        dense_total = 2.0 * nA * (64 * math.ceil(M / 64)) * nF * nB
     elif top == "pure_rows":
         # per launch (one spin side) the compulsory HBM bytes are one read of the
         # input (c~ or its transpose) and one write of the result; the source-row
@@ -312,29 +309,25 @@ def sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma
     else:
         bytes_total = dim * 16.0
         flops_total = 0.0
-    if top != "mixed_gemm":
-        dense_total = None
-    achieved = bytes_total / max(1, n_launch) / per_launch_s / 1e9
-    prof = profile_traffic(f"sigma_{top}_15o7a8b")
+    achieved = bytes_total / stage_s / 1e9
+    # scale a captured launch: of the mixed GEMM by determinants x connected singles (the
+    # elements of Z), of the row kernels by the determinants of two launches (both sides)
+    prof = profile_traffic("sigma_mixed_gemm_14o7a7b" if top == "mixed_gemm" else f"sigma_{top}_15o7a8b")
     traffic = None
     if prof and prof.get("dram_bytes_per_launch") and prof.get("units_per_launch"):
-        # scale the captured launch (15 orbitals) by the determinants one launch covers here
-        units_here = dim / max(1, n_launch)
+        units_here = dim * M if top == "mixed_gemm" else 2 * dim
         traffic = prof["dram_bytes_per_launch"] * units_here / prof["units_per_launch"]
     roof = {"bound": "hbm", "kernel": top, "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": achieved / hbm if hbm else None, "traffic": traffic,
-            "launches_per_sigma": n_launch, "ms_per_launch": per_launch_s * 1e3,
-            "fp64_tflops": flops_total / max(1, n_launch) / per_launch_s / 1e12,
-            "fp64_frac_of_measured_fma_peak": flops_total / max(1, n_launch) / per_launch_s / 1e12 / fp64_peak,
-            "fp64_dense_gemm_tflops": (dense_total / max(1, n_launch) / per_launch_s / 1e12) if dense_total else None,
-            "dense_frac_of_measured_dmma_peak": (dense_total / max(1, n_launch) / per_launch_s / 1e12 / dmma_peak)
-            if dense_total and dmma_peak else None,
-            "note": "dominant kernel of the structured sigma, timed live per launch with CUDA events; achieved = "
-                    "its compulsory HBM bytes per launch / launch time, of the measured HBM copy peak; the mixed GEMM "
-                    "runs as exact byte products on the integer tensor cores, bound by the L1 pipe of its gathers and "
-                    "stores; dense_frac_of_measured_dmma_peak sets the dense FP64 GEMM against the DMMA pipe that it "
-                    "does not use; traffic = ncu dram bytes of a 15-orbital launch of the DMMA kernel (the same rows "
-                    "read and Z written) scaled by determinants per launch"}
+            "launches_per_sigma": n_launch, "ms_per_sigma": t_ms,
+            "fp64_tflops": flops_total / stage_s / 1e12,
+            "fp64_frac_of_measured_fma_peak": flops_total / stage_s / 1e12 / fp64_peak,
+            "note": "dominant stage of the structured sigma, timed live with CUDA events around every launch, summed "
+                    "over one sigma; achieved = its compulsory HBM bytes / that time, of the measured HBM copy peak; "
+                    "fp64_tflops = the connected pairs' operations / that time; the FP64 mixed GEMM runs as exact "
+                    "byte products on the integer tensor cores, bound by the L1 pipe of its gathers and stores (its "
+                    "launches: the byte products, and one for rows left in FP64); traffic = ncu dram bytes of a "
+                    "smaller launch of the same kernel, scaled"}
     return roof, launches
 
 
@@ -450,7 +443,7 @@ def gpu_sigma(args, rank, world, local_rank):
         pk = peaks()
         hbm = pk.get("hbm_gbs")
         tflops = flops / world / (ms * 1e-3) / 1e12
-        roof, launches = sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms, dmma_peak)
+        roof, launches = sigma_roofline(net, pairs, cfg, dim, stages, hbm, fp64_peak, world, ms)
         if launches is None:
             launches = count_launches(step)
         result = {

@@ -81,10 +81,15 @@ constexpr size_t kSmemMax = 227 * 1024;
 template <typename... KArgs>
 inline cudaError_t allow_smem(void (*kern)(KArgs...))
 {
+    const void *k = reinterpret_cast<const void *>(kern);
+    thread_local std::vector<std::pair<const void *, int>> limits;   // asked once a thread: a query costs microseconds
+    for (const auto &l : limits)
+        if (l.first == k) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, l.second);
     cudaFuncAttributes a{};
-    const cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
     if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemMax - a.sharedSizeBytes));
+    limits.emplace_back(k, (int)(kSmemMax - a.sharedSizeBytes));
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limits.back().second);
 }
 
 // Chained launches (programmatic dependent launch): the kernel's CTAs may become

@@ -469,15 +469,15 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
         }
         if (!P->split || m == 0.0) continue;
         lexp[e] = std::ilogb(m) + 1;
-        int n = 0, far = 0;
+        int n = 0, far = 0, least = 0;
         for (int f = 0; f < P->nF; ++f) {
             const double v = std::fabs(row[f]);
             if (v == 0.0) continue;
             ++n;
             far += v < std::ldexp(1.0, lexp[e] - kFarBitsLam);
-            if (v < std::ldexp(1.0, lexp[e] - kLeastBits)) P->split = false;
+            least += v < std::ldexp(1.0, lexp[e] - kLeastBits);
         }
-        if (8 * far > n) P->split = false;
+        if (8 * far > n || 64 * least > n) P->split = false;
     }
 
     // ---- intermediate-string tables ----------------------------------------------

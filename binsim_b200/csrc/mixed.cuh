@@ -86,10 +86,10 @@ int mixed_tc_timeouts(int *count, bool reset);
 // exponent kWideRow, and is left to mixed_dmma_kernel (the line: sigma_split.cu).
 constexpr int kSplitRows = 64;
 constexpr int kWideRow = 0x7fffffff;
-constexpr int kFarBits = 12, kFarBitsLam = 10, kLeastBits = 30;   // of elements: more than 1/8 below, one below
+constexpr int kFarBits = 12, kFarBitsLam = 10, kLeastBits = 30;   // more than 1/8 of the elements below, 1/64 below
 // output rows per pass, 0: no kernel for the shape
 int mixed_split_rows(int nF, int M);
-// rexp: [rows] exponents and the call's flag of waits that gave up
+// rexp: [rows] exponents
 int rows_to_fixed(double *in, int rows, int ld, int *rexp, cudaStream_t s);
 template <typename Ti>
 int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, double *ct, int *rexp, double *Z, int z0, int W, int jbase,

@@ -178,10 +178,10 @@ __device__ __forceinline__ unsigned spread4(unsigned n)
 
 // One CTA per alpha orbit: the rows of its members are walked in the order of
 // the beta lists, all of a row's beta patterns close in time.  256 threads: at 14o
-// 7a+7b a 2000-generator energy and gradient takes 257 ms with them, 263 ms with
-// 512, 299 ms with 1024, and more registers or shared memory to hold fewer CTAs on
-// an SM, or fewer registers to hold more, cost 7-75 %; beta orbits in ascending order
-// instead of sorted by pattern 278 ms.
+// 7a+7b a 2000-generator energy and gradient takes 277 ms with them, 2 % more with
+// 512, 16 % with 1024; more registers or shared memory to hold fewer CTAs on an SM, or
+// fewer registers to hold more, cost 7-75 %, and beta orbits in ascending order
+// instead of sorted by pattern 8 %.
 // BACK: the components in reverse order on l and r, the gradient terms summed
 // into part[CTA][component]; else in order on l.
 template <bool BACK, int NT>

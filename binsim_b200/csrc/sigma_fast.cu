@@ -1506,8 +1506,8 @@ static int run_fast(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastState<Ti> *s
     FastScratch<Ti> &S = st->scratch;
     const int nA = P.nA, nB = P.nB;
     int rc;
-    // c~ (behind it the exponents of its rows as fixed-point numbers and a flag), later c~^T
-    const size_t in_bytes = std::max((size_t)nA * P.ldA * sizeof(T) + ((size_t)nA + 1) * sizeof(int), (size_t)nB * P.ldB * sizeof(T));
+    // c~ (behind it the exponents of its rows as fixed-point numbers), later c~^T
+    const size_t in_bytes = std::max((size_t)nA * P.ldA * sizeof(T) + (size_t)nA * sizeof(int), (size_t)nB * P.ldB * sizeof(T));
     if ((rc = ensure(&S.in, &S.in_n, in_bytes)) != BSIM_OK) return rc;
     if ((rc = ensure(&S.tT, &S.tT_n, (size_t)nB * P.ldB * sizeof(double))) != BSIM_OK) return rc;
     T *in = static_cast<T *>(S.in);

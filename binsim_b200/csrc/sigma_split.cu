@@ -12,7 +12,7 @@
 // word's rounding below 2^-62 of its row's largest element.  FP64 rounds at 2^-53 of a
 // sum's own terms, so the split is as exact only where most elements of a row are not
 // far below its largest: a row of c~ with more than 1/8 of its nonzero elements below
-// 2^-12 of it (of the power of two above it), one below 2^-30 of it, or an infinity or
+// 2^-12 of it (of the power of two above it) or 1/64 below 2^-30, or with an infinity or
 // NaN, stays in FP64 and goes to mixed_dmma_kernel (kWideRow); a Hamiltonian with such a
 // row of Lam (1/8 below 2^-10) does not use the split products at all (fastplan.cu).
 // An output that only the few small elements of an accepted row reach keeps the bound
@@ -37,8 +37,8 @@
 //               matrices, one (column, 8 rows) group per thread;
 //   warp 24     TMEM allocation and, by one lane, the MMA issue.
 // Handoffs and bounded waits as in sigma_tc.cu; a CTA that gives up a wait, and every
-// CTA of the call that starts after it, leaves its row to mixed_dmma_kernel
-// (row_to_fp64).
+// CTA that starts after it and before the next call, leaves its row to
+// mixed_dmma_kernel (row_to_fp64).
 //
 // Bound: the L1 pipe that the producers' gathers, the byte stores and the epilogue's
 // stores share (a slice of 4 K words takes ~3700 cycles, the MMAs of 64 rows 1200 of
@@ -227,10 +227,10 @@ rows_to_fixed_kernel(double *__restrict__ in, int ld, int *__restrict__ rexp)
             atomicAdd(&cnt[2], l);
         }
         __syncthreads();
-        if ((i64)cnt[1] * 8 > cnt[0] || cnt[2] > 0) e = kWideRow;
+        if ((i64)cnt[1] * 8 > cnt[0] || (i64)cnt[2] * 64 > cnt[0]) e = kWideRow;
     }
     if (threadIdx.x == 0) rexp[blockIdx.x] = e;
-    if (blockIdx.x == 0 && threadIdx.x == 0) rexp[gridDim.x] = 0;   // the call's flag of waits that gave up
+    if (blockIdx.x == 0 && threadIdx.x == 0) g_tc_abort = 0;   // of an earlier call (the flag only saves waits)
     if (e == kWideRow) return;   // uniform across the CTA
     for (int i = threadIdx.x; i < ld; i += 256)
         reinterpret_cast<u64 *>(row)[i] = to_word(plain ? (double)row[i] : 0.0, f);
@@ -381,31 +381,38 @@ __device__ __forceinline__ double sum4(int a, int b, int c, int d)
 {
     return unmagic(mad_wide(d, 1, mad_wide(c, 256, mad_wide(b, 65536, mad_wide(a, 16777216, kMagic)))));
 }
-// A CTA's flag and the call's flag of waits that gave up (tc.cuh).
-struct GaveUp {
-    volatile int *cta;
-    int *call;
-};
-// mbar_wait by every lane of a warp, with one answer for all: what follows it is a
-// barrier of the warp or an aligned instruction
-__device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, const GaveUp &gu)
+// mbar_wait with all but its first test out of line: inlined, it takes registers here
+// (0.351 against 0.345 ms at 12o; the kernels of sigma_tc.cu are faster with it inlined).
+__device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag)
 {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, gu.cta, gu.call));
+    return mbar_wait(bar, parity, abort_flag);
+}
+__device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile int *abort_flag)
+{
+    return mbar_try(bar, parity) || wait_slow(bar, parity, abort_flag);
+}
+// wait_phase by every lane of a warp, with one answer for all: what follows it is a
+// barrier of the warp or an aligned instruction
+__device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, volatile int *abort_flag)
+{
+    return __all_sync(0xffffffffu, wait_phase(bar, parity, abort_flag));
 }
 
 // The producers' loop: slice q into A stage q % kStages.
 template <typename Src>
 __device__ __forceinline__ void produce_slices(const SplitLayout &L, unsigned char *smem, uint32_t bar0, int nq, Src &src,
-                                               const GaveUp &gu)
+                                               volatile int *abort_flag)
 {
     const ProdPlace P((int)(threadIdx.x >> 5) - kEpiWarps, (int)(threadIdx.x & 31));
     src.begin(P);
     int st = 0;
     uint32_t empty = 1;   // parity before the first release: passes at once
     auto one = [&](auto set, int q) {
-        if (!wait_all(bar0 + 8u * (uint32_t)(kStages + st), empty, gu)) return false;
+        // a wait that gave up is settled for the warp after the stores, beside its barrier
+        const bool ok = wait_phase(bar0 + 8u * (uint32_t)(kStages + st), empty, abort_flag);
         src.template put<decltype(set)::value>(q, P, smem + L.a + (size_t)st * kStageBytes);
         fence_async_smem();
+        if (!__all_sync(0xffffffffu, ok)) return false;
         warp_arrive(bar0 + 8u * (uint32_t)st);
         if (++st == L.stages) { st = 0; empty ^= 1u; }
         return true;
@@ -439,7 +446,7 @@ __device__ __forceinline__ void issue_planes(const SplitLayout &L, uint32_t sbas
 template <typename Src>
 __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned char *smem, uint32_t sbase, uint32_t tmem,
                                             int ncb, int jm, double *zrow, int zrows, Src &src,
-                                            const GaveUp &gu, bool drop)
+                                            volatile int *abort_flag, bool drop)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bar0 = sbase + L.bars;   // afull[S], aempty[S], dfull[2], dempty[2], done
@@ -452,7 +459,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
     const int n0 = half_rows(jm, 0), n1 = half_rows(jm, 1), nh = n1 ? 2 : 1, nu = ncb * nh;
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kProdWarps) {
-        if (!drop) produce_slices(L, smem, bar0, ncb * nsl, src, gu);
+        if (!drop) produce_slices(L, smem, bar0, ncb * nsl, src, abort_flag);
     } else if (warp == kMmaWarp) {
         // ---- MMA issue (one elected lane).  With a chunk's slices all in stages, half by
         // half, so that one half's accumulator is read out during the other's MMAs; else
@@ -473,13 +480,13 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
                     st = st0;
                     full = full0;
                     // the accumulator's previous part was read out
-                    if (so == 0 && u >= 2 && !wait_all(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), gu)) {
+                    if (so == 0 && u >= 2 && !wait_all(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), abort_flag)) {
                         ok = false;
                         break;
                     }
                     for (int si = 0; si < nin; ++si) {
                         const int s = so * nin + si;
-                        if (h == 0 && !wait_all(afull(st), full, gu)) { ok = false; break; }
+                        if (h == 0 && !wait_all(afull(st), full, abort_flag)) { ok = false; break; }
                         tc_fence_after();
                         if (lead) {
                             issue_planes(L, sbase, st, s, boff, n, tmem + (uint32_t)(ND * n0 * acc));
@@ -495,7 +502,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
             }
         if (lead) umma_commit(done);   // every issued MMA has completed before TMEM is freed
         __syncwarp();
-        if (lane == 0) mbar_wait_drain(done, 0u, gu.call);
+        if (lane == 0) mbar_wait_drain(done, 0u);
         __syncwarp();
     } else if (warp < kEpiWarps) {
         // ---- epilogue: half of the part's rows per warp, eight at a time ----
@@ -503,7 +510,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
         const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         for (int u = 0; u < nu; ++u) {
             const int c = u / nh, h = u % nh, acc = u & 1;
-            if (!wait_all(dfull(acc), (uint32_t)((u >> 1) & 1), gu)) break;
+            if (!wait_all(dfull(acc), (uint32_t)((u >> 1) & 1), abort_flag)) break;
             tc_fence_after();
             const int n = h ? n1 : n0, e0 = (warp >> 2) * (n / 2), e1 = min(e0 + n / 2, jm - kHalf * h);
             const uint32_t base = lanes + (uint32_t)(ND * n0 * acc);
@@ -578,7 +585,8 @@ __device__ __forceinline__ uint32_t split_cols(int cols) { return cols > 256 ? 5
 // A row's words back to FP64, and the row to mixed_dmma_kernel: the end of a CTA whose
 // waits gave up, so that a stalled device costs time and never a result.  The elements
 // are those of the words, within 2^-63 of the row's largest.
-__device__ void row_to_fp64(u64 *row, int ld, int e, int *rexp)
+// Out of line: inlined, it takes the kernel's registers (72.0 against 67.9 ms at 16o).
+__device__ __noinline__ void row_to_fp64(u64 *row, int ld, int e, int *rexp)
 {
     const Pow2 f(e - kBits);
     for (int i = threadIdx.x; i < ld; i += kThreads)
@@ -603,10 +611,9 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, u64 *ct,
     __shared__ volatile int abort_flag;
     __shared__ int skip_all;
     const int a = blockIdx.x, aexp = rexp[a];
-    int *call_flag = rexp + P.nA;
     u64 *row = ct + (i64)a * P.ldA;
     if (aexp == kWideRow) return;   // uniform across the CTA: mixed_dmma_kernel computes the row
-    if (threadIdx.x == 0) skip_all = *(volatile int *)call_flag;
+    if (threadIdx.x == 0) skip_all = *(volatile int *)&g_tc_abort;
     __syncthreads();
     if (skip_all) {   // an earlier CTA gave up a wait
         row_to_fp64(row, P.ldA, aexp, rexp + a);
@@ -633,9 +640,10 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, u64 *ct,
     src.nsl = L.kp / kKS;
     src.nq = ncb * src.nsl;
     split_pipeline(L, smem, sbase, tmem, ncb, jm, zchunk(Z, a, P.M, W, 0) + jbase * kM, P.M, src,
-                   GaveUp{&abort_flag, call_flag}, a == drop);
+                   &abort_flag, a == drop);
     split_end(tmem, cols);
-    if (abort_flag) row_to_fp64(row, P.ldA, aexp, rexp + a);   // uniform: written before split_end's barrier
+    if (abort_flag)   // uniform: written before split_end's barrier
+        row_to_fp64(ct + (i64)a * P.ldA, P.ldA, rexp[a], rexp + a);
 }
 
 }  // namespace

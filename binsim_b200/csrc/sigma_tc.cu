@@ -63,8 +63,6 @@ constexpr int kMixKSGrow = 40;            // the same, row read from global memo
 constexpr int kMixStages = 2;             // its A stages
 constexpr int kRiStages = 2, kRiRing = 4; // the intermediate product's A stages and copy-ring slots
 
-__device__ int g_tc_abort;   // set with the first wait that gives up: later CTAs return at once
-
 // two N-column accumulators, allocated as a power of 2 of at least 32 columns
 template <int N>
 constexpr uint32_t tmem_cols() { return N <= 16 ? 32u : N <= 32 ? 64u : N <= 64 ? 128u : 256u; }
@@ -256,7 +254,7 @@ __device__ __forceinline__ void tc_pipeline(const TcLayout &L, unsigned char *sm
     if (warp >= 4 && warp < 4 + kTcProdWarps) {
         // ---- producers ----
         auto free_stage = [&](int t) -> bool {
-            return t < S || mbar_wait(aempty(t % S), (uint32_t)(((t / S) - 1) & 1), abort_flag, &g_tc_abort);
+            return t < S || mbar_wait(aempty(t % S), (uint32_t)(((t / S) - 1) & 1), abort_flag);
         };
         src.setup(warp - 4, lane);
         src.begin(nq);
@@ -272,12 +270,12 @@ __device__ __forceinline__ void tc_pipeline(const TcLayout &L, unsigned char *sm
             bool ok = true;
             for (int c = 0; c < ncb && ok; ++c) {
                 const int dbuf = c & 1;
-                if (c >= 2 && !mbar_wait(dempty(dbuf), (uint32_t)(((c >> 1) - 1) & 1), abort_flag, &g_tc_abort)) break;
+                if (c >= 2 && !mbar_wait(dempty(dbuf), (uint32_t)(((c >> 1) - 1) & 1), abort_flag)) break;
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)dbuf * N;
                 for (int s = 0; s < nsl; ++s) {
                     const int q = c * nsl + s, st = q % S;
-                    if (!mbar_wait(afull(st), (uint32_t)((q / S) & 1), abort_flag, &g_tc_abort)) { ok = false; break; }
+                    if (!mbar_wait(afull(st), (uint32_t)((q / S) & 1), abort_flag)) { ok = false; break; }
                     tc_fence_after();
                     const int f0 = s * KS, nks = (min(KS, L.kp8 - f0) + 7) / 8;
                     const uint32_t ah = sbase + L.ah + (uint32_t)st * L.abytes, al = sbase + L.al + (uint32_t)st * L.abytes;
@@ -297,7 +295,7 @@ __device__ __forceinline__ void tc_pipeline(const TcLayout &L, unsigned char *sm
                 if (ok) umma_commit(dfull(dbuf));
             }
             umma_commit(done);   // every issued MMA has completed before TMEM is freed
-            mbar_wait_drain(done, 0u, &g_tc_abort);
+            mbar_wait_drain(done, 0u);
         }
         __syncwarp();
     } else if (warp < 4) {
@@ -305,7 +303,7 @@ __device__ __forceinline__ void tc_pipeline(const TcLayout &L, unsigned char *sm
         for (int c = 0; c < ncb; ++c) {
             const int dbuf = c & 1;
             // one answer for the warp: the tensor-memory loads below are aligned
-            if (!__all_sync(0xffffffffu, mbar_wait(dfull(dbuf), (uint32_t)((c >> 1) & 1), abort_flag, &g_tc_abort))) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(dfull(dbuf), (uint32_t)((c >> 1) & 1), abort_flag))) break;
             tc_fence_after();
             const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)dbuf * N;
             float *zb = zrow + (i64)c * zrows * kTcM + warp * 32 + lane;

@@ -16,6 +16,7 @@ constexpr unsigned kTcSuspendNs = 20000;                // longest sleep in one 
 constexpr uint32_t kCoreBytes = 128;      // one core matrix: 8 rows x 16 bytes
 
 __device__ int g_tc_timeouts;   // waits that gave up
+__device__ int g_tc_abort;      // set with the first of them: later CTAs do not start their waits
 
 __host__ __device__ inline uint32_t align128(uint32_t x) { return (x + 127u) & ~127u; }
 
@@ -55,11 +56,10 @@ __device__ __forceinline__ unsigned long long global_ns()
 }
 
 // Bounded wait for the phase of the given parity; false when the CTA aborts
-// (its own wait gave up, another wait of the CTA did, or another CTA's did, which sets
-// *abort_all).
+// (its own wait gave up, another wait of the CTA did, or another CTA's did).
 // The flags and the clock are read after every kTcCheck tests that came back without
 // the phase.
-__device__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int *abort_flag, int *abort_all)
+__device__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int *abort_flag)
 {
     if (mbar_try(a, parity)) return true;
     const unsigned long long t0 = global_ns();
@@ -67,25 +67,25 @@ __device__ bool mbar_wait(uint32_t a, uint32_t parity, volatile int *abort_flag,
         if (mbar_try(a, parity)) return true;
         if (i % kTcCheck) continue;
         if (*abort_flag) return false;
-        if (*(volatile int *)abort_all) { *abort_flag = 1; return false; }
+        if (*(volatile int *)&g_tc_abort) { *abort_flag = 1; return false; }
         if (i >= kTcMinSpins && global_ns() - t0 > kTcWaitNs) break;
     }
     *abort_flag = 1;
-    atomicExch(abort_all, 1);
+    atomicExch(&g_tc_abort, 1);
     atomicAdd(&g_tc_timeouts, 1);
     return false;
 }
 
 // Bounded wait that ignores the abort flags: the wait for this CTA's own MMAs
 // before its tensor memory is freed.
-__device__ void mbar_wait_drain(uint32_t a, uint32_t parity, int *abort_all)
+__device__ void mbar_wait_drain(uint32_t a, uint32_t parity)
 {
     const unsigned long long t0 = global_ns();
     for (long i = 0; i < kTcSpinCap; ++i) {
         if (mbar_try(a, parity)) return;
         if (i >= kTcMinSpins && global_ns() - t0 > kTcWaitNs) break;
     }
-    atomicExch(abort_all, 1);
+    atomicExch(&g_tc_abort, 1);
     atomicAdd(&g_tc_timeouts, 1);
 }
 

@@ -17,7 +17,7 @@
  *
  * Thread safety: a basis handle owns reusable device scratch, so calls that
  * share one basis handle must be issued from one host thread / one stream at
- * a time.
+ * a time.  One network may serve several threads that use a basis each.
  */
 #ifndef BINSIM_CUOTF_H
 #define BINSIM_CUOTF_H
@@ -159,7 +159,7 @@ int64_t bsim_network_ngs(void *net);
  * single-single excitations go through fixed-point words of 62 bits below the
  * largest element of an alpha row of src, multiplied exactly.  A row keeps FP64
  * elements and sums when more than 1/8 of its nonzero elements lie below 2^-12
- * of that largest one, any below 2^-30 of it, or it holds an infinity or NaN.
+ * of that largest one, 1/64 below 2^-30 of it, or it holds an infinity or NaN.
  * So the error of an output is that of FP64 sums of its own terms, except for an
  * output that only the few small elements of a row reach: there it is up to
  * 2^-57 of (the row's largest element) x (the largest integral) a term. */

@@ -68,7 +68,7 @@ def test_two_threads_one_network(cuda, oracle, blocked):
 
 
 def test_bases_in_turn_make_no_new_plans(cuda):
-    """Symmetry blocks and complex sigma: the plans of two irreps stay while both bases live, and go with them."""
+    """Symmetry blocks and complex sigma: the plans of two irreps stay while both bases live."""
     from binsim_b200 import cuotf
     from binsim_b200.cuotf import lib
     ham, w, kw = _setup(True)
@@ -89,6 +89,30 @@ def test_bases_in_turn_make_no_new_plans(cuda):
     n = lib().bsim_device_alloc_count()
     both()
     assert lib().bsim_device_alloc_count() == n
+
+
+def test_a_plan_goes_with_its_basis(cuda):
+    """Lists of the complex sigma at 10o 5+5 (tens of megabytes) are given back when the basis is destroyed, the network
+    still alive."""
+    from binsim_b200 import cuotf, network as nw
+    ham = nw.hamiltonian_network(10, seed=1, native=True)
+    Z = cuotf.CuNetworkC64(ham, ham.flat_wa.astype(complex), ham.flat_wb.astype(complex))
+    z = cuda.ones(252 * 252, dtype=cuda.complex128, device="cuda")
+    u = cuda.empty_like(z)
+
+    def free():
+        cuda.cuda.synchronize()
+        return cuda.cuda.mem_get_info()[0]
+    for _ in range(2):   # the first round also loads the kernels
+        before = free()
+        B = cuotf.CuBasis(10, 5, 5)
+        f = cuotf.CuOTFC64(B, Z)
+        f.hvec(z, u)
+        used = before - free()
+        del f
+        B.close()
+        left = before - free()
+    assert used > 8e6 and left < 4e6, (used, left)
 
 
 def test_shapes_of_two_threads(cuda):

@@ -90,6 +90,17 @@ struct StrIndex {
 
 }  // namespace
 
+// The split kernel's gather table (MixedArgs): gidx as byte offsets by column, F to whole
+// slices of 32.  On the device: made by the host and uploaded it cost every plan more.
+__global__ void split_offsets_kernel(const int *__restrict__ gidx, int nF, int nFp, int ldG, unsigned none,
+                                     unsigned *__restrict__ goff)
+{
+    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < (i64)ldG * nFp; i += (i64)gridDim.x * blockDim.x) {
+        const int f = (int)(i % nFp), g = f < nF ? gidx[(i64)f * ldG + i / nFp] : -1;
+        goff[i] = g < 0 ? none : (unsigned)(g >> 1) * 8u | (unsigned)(g & 1) << 31;
+    }
+}
+
 template <typename Ti>
 int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
 {
@@ -457,9 +468,8 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
             }
     }
 
-    std::vector<int> &lexp = P->lexp;
-    lexp.assign(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
-    P->split = true;
+    std::vector<int> lexp(P->nE, -2000);   // smallest e with |Lam| < 2^e; a row of zeros: -2000
+    P->split = P->nE > 0 && P->nF > 0 && mixed_split_rows(P->nF, P->M) > 0;
     for (int e = 0; e < P->nE && P->split; ++e) {
         const double *row = &P->Lam[(size_t)e * P->nF];
         double m = 0.0;
@@ -549,10 +559,13 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     }
 
     // ---- upload -------------------------------------------------------------------
+    const int nFp = (P->nF + 31) & ~31;
+    const size_t goff_n = (size_t)P->ldG * nFp;
     auto bytes = [](size_t n, size_t sz) { return ((std::max<size_t>(n, 1) * sz) + 255) & ~size_t(255); };
     size_t tot = bytes(nA, sizeof(Ti)) + bytes(nB, sizeof(Ti)) + bytes(nA, 8) + bytes(PAd.size(), 8) +
                  bytes(PBd.size(), 8) + 2 * bytes(P->nE, 8) + 2 * bytes(P->Lam.size(), 8) + bytes(gidx.size(), 4) +
-                 bytes(P->residual.size(), 4) + bytes(P->residual.size() + 1, 16);
+                 bytes(P->residual.size(), 4) + bytes(P->residual.size() + 1, 16) +
+                 (P->split ? bytes(goff_n, 4) + bytes(lexp.size(), 4) : 0);
     for (int li = 0; li < 3; ++li)
         tot += 2 * bytes(csr[li].cptr.size(), 8) + bytes(csr[li].cent.size(), sizeof(CEnt)) +
                bytes(csr[li].tent.size(), sizeof(TEnt)) + bytes(sh[li == 0 ? 0 : 1].ctab.size(), 8) +
@@ -579,6 +592,12 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
     std::vector<float> lam32(P->Lam.begin(), P->Lam.end());
     P->d_Lam32 = put(lam32);
     P->d_gidx = put(gidx);
+    if (P->split) {
+        unsigned *goff = P->arena.template take<unsigned>(goff_n);
+        split_offsets_kernel<<<148, 256>>>(P->d_gidx, P->nF, nFp, P->ldG, (unsigned)nB * 8u, goff);
+        P->d_goff = goff;
+        P->d_lexp = put(lexp);
+    }
     for (int li = 0; li < 3; ++li) {
         CSRHost &C = csr[li];
         if (li == 2 && !ri_on[1]) continue;

@@ -110,8 +110,9 @@ struct FastPlan {
     const float *d_Lam32 = nullptr;
     const double *d_PBdT = nullptr;    // [rank_d x ldA] beta diagonal factors, transposed
     const int *d_gidx = nullptr;       // [nF x ldG] (rank(b^F) << 1 | sign) or -1
-    std::vector<int> lexp;             // [nE] exponent above a row of Lam
-    bool split = false;                // the rows of Lam suit the split products (sigma_split.cu)
+    const unsigned *d_goff = nullptr;  // the same as byte offsets, by column (MixedArgs), when split
+    const int *d_lexp = nullptr;       // [nE] exponent above a row of Lam, when split
+    bool split = false;                // the sizes and the rows of Lam suit the split products (sigma_split.cu)
     const int *d_resid = nullptr;      // residual group plan (for the generic kernel)
     const int4 *d_resid_chunks = nullptr;
     int n_resid_chunks = 0;

@@ -1076,9 +1076,8 @@ template <typename Ti>
 struct FastScratch {
     void *in = nullptr, *tT = nullptr, *Z = nullptr;
     size_t in_n = 0, tT_n = 0, z_n = 0;
-    void *split = nullptr;   // split_tables
     ~FastScratch() {
-        for (void *p : {in, tT, Z, split})
+        for (void *p : {in, tT, Z})
             if (p) cudaFree(p);
     }
 };
@@ -1286,49 +1285,6 @@ static int mixed_split(const FastPlan<Ti> &P)
     return mixed_split_rows(P.nF, P.M);
 }
 
-// The split kernel's tables (MixedArgs): gidx as byte offsets by column, F to whole
-// slices of 32, and the exponents of Lam's rows.  Made with its first call, on the
-// device: most handles of small bases never need them.  False: none and no room, or
-// inside a stream capture; the DMMA kernel serves the call.
-__global__ void split_offsets_kernel(const int *__restrict__ gidx, int nF, int nFp, int ldG, unsigned none,
-                                     unsigned *__restrict__ goff)
-{
-    for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < (i64)ldG * nFp; i += (i64)gridDim.x * blockDim.x) {
-        const int f = (int)(i % nFp), g = f < nF ? gidx[(i64)f * ldG + i / nFp] : -1;
-        goff[i] = g < 0 ? none : (unsigned)(g >> 1) * 8u | (unsigned)(g & 1) << 31;
-    }
-}
-template <typename Ti>
-static int split_tables(const FastPlan<Ti> &P, FastScratch<Ti> &S, MixedArgs &ma, cudaStream_t s, bool *have)
-{
-    *have = false;
-    const int nFp = (P.nF + 31) & ~31;
-    const size_t n = (size_t)P.ldG * nFp;
-    if (!S.split) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        BSIM_CUDA(cudaStreamIsCapturing(s, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return BSIM_OK;
-        unsigned *p = nullptr;
-        const cudaError_t e = dmalloc(&p, n * 4 + P.lexp.size() * 4);
-        if (e == cudaErrorMemoryAllocation) { (void)cudaGetLastError(); return BSIM_OK; }
-        if (e != cudaSuccess) return cuda_status(e, "split product tables");
-        cudaError_t e2 = cudaMemcpy(p + n, P.lexp.data(), P.lexp.size() * 4, cudaMemcpyHostToDevice);
-        if (e2 == cudaSuccess) {
-            split_offsets_kernel<<<148, 256, 0, s>>>(P.d_gidx, P.nF, nFp, P.ldG, (unsigned)P.nB * 8u, p);
-            e2 = cudaGetLastError();
-        }
-        if (e2 != cudaSuccess) {
-            cudaFree(p);
-            return cuda_status(e2, "split product tables");
-        }
-        S.split = p;
-    }
-    ma.goff = static_cast<const unsigned *>(S.split);
-    ma.lexp = reinterpret_cast<const int *>(ma.goff + n);
-    *have = true;
-    return BSIM_OK;
-}
-
 template <typename Ti, typename T, int EPT>
 static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> &S, T *ct, double *dst,
                         int c0, int c1, cudaStream_t s, StageTimer *tm)
@@ -1338,15 +1294,13 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
     int rc = z_slot(&S.Z, &S.z_n, S.tT, S.tT_n, per_col, c1 - c0, &z);
     if (rc != BSIM_OK) return rc;
     MixedArgs ma{P.nA, P.nB, P.nE, P.nF, P.M, P.ldA, P.ldG, c1, P.d_Emask, P.d_mA,
-                 sizeof(T) == 8 ? (const void *)P.d_Lam : (const void *)P.d_Lam32, P.d_gidx, nullptr, nullptr};
+                 sizeof(T) == 8 ? (const void *)P.d_Lam : (const void *)P.d_Lam32, P.d_gidx, P.d_goff, P.d_lexp};
     if constexpr (sizeof(T) == 8) {
         const int rows = mixed_split(P);
         const bool on_chip = mixed_dmma_smem(P.ldA, P.nF, false) <= std::min(kSmemMax, mixed_row_limit());
         const size_t smem = mixed_dmma_smem(P.ldA, P.nF, !on_chip);
         auto kern = on_chip ? mixed_dmma_kernel<Ti, false> : mixed_dmma_kernel<Ti, true>;
-        bool split = false;
-        if (rows > 0 && smem <= kSmemMax && (rc = split_tables(P, S, ma, s, &split)) != BSIM_OK) return rc;
-        if (split) {   // split products; nothing reads a converted row in floating point after this
+        if (rows > 0 && smem <= kSmemMax) {   // split products; nothing reads a converted row in floating point after this
             BSIM_CUDA(allow_smem(kern));
             int *rexp = reinterpret_cast<int *>(ct + (size_t)P.nA * P.ldA);   // behind the rows (run_fast)
             double *Z = static_cast<double *>(z.p);

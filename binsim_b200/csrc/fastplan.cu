@@ -176,10 +176,18 @@ int build_fast_plan(const DevBasis<Ti> *B, const DevNet<Ti> *N, FastPlan<Ti> *P)
             const double *cw = w + (side == 0 ? G.wb_off : G.wa_off);
             // the frame flips the column factor by (-1)^{popc(col & M)}
             const u64 cm = side == 0 ? mask_above_odd(rowx, norb) : mask_below_odd(rowx, norb);
+            // masks that are empty or full in the frame give every string the same sign
+            // (those of a pure double): one column tells the factor
+            const u64 full = (1ull << norb) - 1;
+            bool one = true;
+            for (int q = 0; q < cnz; ++q) {
+                const u64 m = ((u64)cz[q] ^ cm) & full;
+                one = one && (m == 0 || m == full);
+            }
             std::vector<double> col((size_t)G.rank * ncol);
             bool constant = true;
             for (int r = 0; r < G.rank; ++r)
-                for (int c = 0; c < ncol; ++c) {
+                for (int c = 0; c < (one ? 1 : ncol); ++c) {
                     double v = phase_r((u64)colstr[c], cz, cnz, cw, r, cm);
                     col[(size_t)r * ncol + c] = v;
                     if (std::fabs(v - col[(size_t)r * ncol]) > 1e-13 * std::max(1.0, std::fabs(col[(size_t)r * ncol])))

@@ -635,14 +635,16 @@ mixed_gemm_kernel(const MixedArgs P, const Ti *__restrict__ astr, const T *__res
 // synchronise inside the loop.  Lam_conn (the A fragments, read by every warp)
 // is staged once per CTA with rows g and g + 8 of each 16-row tile side by
 // side, so a lane's two A elements of a K step are one 16-byte load.
-// rexp (null: every row): the rows that the split products leave (kWideRow).
+// WIDE: the rows that the split products leave (kWideRow in rexp) instead of every row,
+// one CTA each.  They are often a few, and a CTA takes 0.17 ms for a row of 20o 3+3: the
+// grid shares their column chunks.
 constexpr int kDmmaLS = 34;   // double2 per F row: 32 + 2 (2 mod 8: conflict-free 16-byte fragment loads)
 inline size_t mixed_dmma_smem(int ldA, int nF, bool grow)
 {
     return (grow ? 0 : (size_t)ldA * 8) + (size_t)((nF + 31) & ~31) * kDmmaLS * 16 + 2 * kMaxConn * 4;
 }
 
-template <typename Ti, bool GROW>
+template <typename Ti, bool GROW, bool WIDE>
 __global__ void __launch_bounds__(512, 1)
 mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *__restrict__ ct,
                   double *__restrict__ Z, int z0, int W, int jbase, const int *__restrict__ rexp)
@@ -656,9 +658,52 @@ mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *
     double2 *lam = reinterpret_cast<double2 *>(srow + (GROW ? 0 : P.ldA));   // [Kp][kDmmaLS], rows past K zero
     int *conn = reinterpret_cast<int *>(lam + (size_t)Kp * kDmmaLS);        // [kMaxConn]
     int *sgn = conn + kMaxConn;                                              // [kMaxConn]
-    __shared__ int wcnt[NT / 32], cnt;
-    for (int a = blockIdx.x; a < P.nA; a += gridDim.x) {
-        if (rexp && rexp[a] != kWideRow) continue;   // uniform: the split kernel computed this source row
+    __shared__ int wcnt[NT / 32], cnt, wide_row;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int zend = min(P.cend, z0 + W);
+    const int ncb = (zend - z0 + kMixCols - 1) / kMixCols;
+    // items: (row, segment of the column chunks); of rexp's rows, this thread counts a
+    // stretch and finds those of them that an item asks for
+    int items = P.nA, nseg = 1, first = 0, last = 0, before = 0, mine = 0;
+    if constexpr (WIDE) {
+        const int per = (P.nA + NT - 1) / NT;
+        first = min(P.nA, (int)threadIdx.x * per);
+        last = min(P.nA, first + per);
+        for (int i = first; i < last; ++i) mine += rexp[i] == kWideRow;
+        int inc = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
+        }
+        if (lane == 31) wcnt[wid] = inc;
+        __syncthreads();
+        int total = 0;
+        for (int i = 0; i < NT / 32; ++i) {
+            if (i < wid) before += wcnt[i];
+            total += wcnt[i];
+        }
+        before += inc - mine;
+        __syncthreads();
+        if (total == 0) return;   // uniform
+        nseg = max(1, min((int)gridDim.x / total, ncb));
+        items = total * nseg;
+    }
+    for (int item = blockIdx.x; item < items; item += gridDim.x) {
+        int a = item;
+        if constexpr (WIDE) {
+            const int k = item / nseg - before;   // the k-th of this thread's rows
+            if (k >= 0 && k < mine)
+                for (int i = first, n = 0; i < last; ++i)
+                    if (rexp[i] == kWideRow && n++ == k) wide_row = i;
+            __syncthreads();
+            a = wide_row;
+        }
+        int c_lo = 0, c_hi = ncb;
+        if constexpr (WIDE) {
+            c_lo = (int)((i64)ncb * (item % nseg) / nseg);
+            c_hi = (int)((i64)ncb * (item % nseg + 1) / nseg);
+        }
         const int m = connected_excitations<NT>(P, (u64)astr[a], conn, sgn, wcnt, &cnt);
         const int jm = min(64, m - jbase);   // output rows of this pass
         if (jm <= 0) {                       // uniform across the CTA
@@ -685,17 +730,14 @@ mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *
             lam[i] = v;
         }
         __syncthreads();
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
         const int nrb = (jm + 15) >> 4;   // 16-row tiles holding connected rows
-        const int zend = min(P.cend, z0 + W);
-        const int ncb = (zend - z0 + kMixCols - 1) / kMixCols;
         const int nfc = (K + 31) / 32;
-        const int nsteps = ncb * nfc;
+        const int nsteps = (c_hi - c_lo) * nfc;
         const int col = 8 * wid + g;     // this lane's B column within a chunk
         int gp[8];
         double gv[GROW ? 8 : 1];
         auto load = [&](int step) {
-            const int cb = z0 + (step / nfc) * kMixCols, f0 = (step % nfc) * 32;
+            const int cb = z0 + (c_lo + step / nfc) * kMixCols, f0 = (step % nfc) * 32;
             const int *gb = P.gidx + (i64)(f0 + t) * P.ldG + cb + col;
 #pragma unroll
             for (int i = 0; i < 8; ++i) gp[i] = f0 + 4 * i + t < K ? __ldg(gb + (i64)(4 * i) * P.ldG) : -1;
@@ -709,7 +751,7 @@ mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *
         for (int rb = 0; rb < 4; ++rb) c[rb][0] = c[rb][1] = c[rb][2] = c[rb][3] = 0.0;
         if (nsteps > 0) load(0);
         for (int step = 0; step < nsteps; ++step) {
-            const int cbi = step / nfc, fci = step % nfc;
+            const int cbi = c_lo + step / nfc, fci = step % nfc;
             const int f0 = fci * 32, nk = (min(32, K - f0) + 3) >> 2;
             double x[8];
 #pragma unroll
@@ -744,7 +786,8 @@ mixed_dmma_kernel(const MixedArgs P, const Ti *__restrict__ astr, const double *
                 }
             }
         }
-        __syncthreads();   // the shared arrays are free for the next row
+        if constexpr (!WIDE) return;
+        __syncthreads();   // the shared arrays are free for the next item
     }
 }
 
@@ -1299,7 +1342,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
         const int rows = mixed_split(P);
         const bool on_chip = mixed_dmma_smem(P.ldA, P.nF, false) <= std::min(kSmemMax, mixed_row_limit());
         const size_t smem = mixed_dmma_smem(P.ldA, P.nF, !on_chip);
-        auto kern = on_chip ? mixed_dmma_kernel<Ti, false> : mixed_dmma_kernel<Ti, true>;
+        auto kern = on_chip ? mixed_dmma_kernel<Ti, false, true> : mixed_dmma_kernel<Ti, true, true>;
         if (rows > 0 && smem <= kSmemMax) {   // split products; nothing reads a converted row in floating point after this
             BSIM_CUDA(allow_smem(kern));
             int *rexp = reinterpret_cast<int *>(ct + (size_t)P.nA * P.ldA);   // behind the rows (run_fast)
@@ -1311,7 +1354,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
                     STAGE(tm, 3, s, rc = mixed_gemm_split<Ti>(ma, P.d_astr, ct, rexp, Z, z0, (int)z.w, jb, rows, s));
                     if (rc != BSIM_OK) return rc;
                 }
-                for (int jb = 0; jb < P.M; jb += 64)   // rows left in FP64: one CTA per SM looks for them
+                for (int jb = 0; jb < P.M; jb += 64)   // rows left in FP64: one CTA per SM shares them
                     STAGE(tm, 3, s, (launch_chained(kern, std::min(P.nA, 148), 512, smem, s, ma, P.d_astr, ct, Z, z0,
                                                    (int)z.w, jb, (const int *)rexp)));
                 dim3 g(P.nA, (unsigned)((std::min<size_t>(z.w, c1 - z0) + kRowChunk - 1) / kRowChunk));
@@ -1358,7 +1401,7 @@ static int launch_mixed(const DevBasis<Ti> *B, FastPlan<Ti> &P, FastScratch<Ti> 
             const bool on_chip = mixed_dmma_smem(P.ldA, P.nF, false) <= std::min(kSmemMax, mixed_row_limit());
             const size_t smem = mixed_dmma_smem(P.ldA, P.nF, !on_chip);
             if (smem <= kSmemMax) {
-                auto kern = on_chip ? mixed_dmma_kernel<Ti, false> : mixed_dmma_kernel<Ti, true>;
+                auto kern = on_chip ? mixed_dmma_kernel<Ti, false, false> : mixed_dmma_kernel<Ti, true, false>;
                 BSIM_CUDA(allow_smem(kern));
                 const int passes = (P.M + 63) / 64;
                 T *Z = static_cast<T *>(z.p);

@@ -381,25 +381,30 @@ __device__ __forceinline__ double sum4(int a, int b, int c, int d)
 {
     return unmagic(mad_wide(d, 1, mad_wide(c, 256, mad_wide(b, 65536, mad_wide(a, 16777216, kMagic)))));
 }
-// mbar_wait with all but its first test out of line: inlined, it takes registers here
-// (0.351 against 0.345 ms at 12o; the kernels of sigma_tc.cu are faster with it inlined).
+// mbar_wait with all but its first test out of line where a chunk's slices all have
+// stages (FITS): inlined it takes registers (351 against 343 us at 12o, 799 / 779 at
+// 13o 7+5).  Slice by slice the waits are longer and the call costs more (20o 3+3: 892
+// us with it, 816 inlined and in an instance of its own).
 __device__ __noinline__ bool wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag)
 {
     return mbar_wait(bar, parity, abort_flag);
 }
+template <bool FITS>
 __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity, volatile int *abort_flag)
 {
-    return mbar_try(bar, parity) || wait_slow(bar, parity, abort_flag);
+    if constexpr (FITS) return mbar_try(bar, parity) || wait_slow(bar, parity, abort_flag);
+    else return mbar_wait(bar, parity, abort_flag);
 }
 // wait_phase by every lane of a warp, with one answer for all: what follows it is a
 // barrier of the warp or an aligned instruction
+template <bool FITS>
 __device__ __forceinline__ bool wait_all(uint32_t bar, uint32_t parity, volatile int *abort_flag)
 {
-    return __all_sync(0xffffffffu, wait_phase(bar, parity, abort_flag));
+    return __all_sync(0xffffffffu, wait_phase<FITS>(bar, parity, abort_flag));
 }
 
 // The producers' loop: slice q into A stage q % kStages.
-template <typename Src>
+template <bool FITS, typename Src>
 __device__ __forceinline__ void produce_slices(const SplitLayout &L, unsigned char *smem, uint32_t bar0, int nq, Src &src,
                                                volatile int *abort_flag)
 {
@@ -409,7 +414,7 @@ __device__ __forceinline__ void produce_slices(const SplitLayout &L, unsigned ch
     uint32_t empty = 1;   // parity before the first release: passes at once
     auto one = [&](auto set, int q) {
         // a wait that gave up is settled for the warp after the stores, beside its barrier
-        const bool ok = wait_phase(bar0 + 8u * (uint32_t)(kStages + st), empty, abort_flag);
+        const bool ok = wait_phase<FITS>(bar0 + 8u * (uint32_t)(kStages + st), empty, abort_flag);
         src.template put<decltype(set)::value>(q, P, smem + L.a + (size_t)st * kStageBytes);
         fence_async_smem();
         if (!__all_sync(0xffffffffu, ok)) return false;
@@ -443,7 +448,7 @@ __device__ __forceinline__ void issue_planes(const SplitLayout &L, uint32_t sbas
 }
 
 // Parts u = chunk * (parts per chunk) + half, accumulator u % 2.
-template <typename Src>
+template <bool FITS, typename Src>
 __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned char *smem, uint32_t sbase, uint32_t tmem,
                                             int ncb, int jm, double *zrow, int zrows, Src &src,
                                             volatile int *abort_flag, bool drop)
@@ -459,14 +464,16 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
     const int n0 = half_rows(jm, 0), n1 = half_rows(jm, 1), nh = n1 ? 2 : 1, nu = ncb * nh;
 
     if (warp >= kEpiWarps && warp < kEpiWarps + kProdWarps) {
-        if (!drop) produce_slices(L, smem, bar0, ncb * nsl, src, abort_flag);
+        if (!drop) produce_slices<FITS>(L, smem, bar0, ncb * nsl, src, abort_flag);
     } else if (warp == kMmaWarp) {
         // ---- MMA issue (one elected lane).  With a chunk's slices all in stages, half by
         // half, so that one half's accumulator is read out during the other's MMAs; else
         // slice by slice ----
         const bool lead = elect_lane();
-        const int nslow = nsl > L.stages ? nsl : 1;   // slices outside the halves' loop
-        const int nin = nsl / nslow;                  // and inside
+        // slices outside the halves' loop (1 where they fit; a constant there made the
+        // kernel take 355 us at 12o) and inside
+        const int nslow = !FITS || nsl > L.stages ? nsl : 1;
+        const int nin = FITS ? nsl / nslow : 1;
         bool ok = true;
         int st0 = 0;
         uint32_t full0 = 0;   // stage and parity of the next slice
@@ -480,13 +487,13 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
                     st = st0;
                     full = full0;
                     // the accumulator's previous part was read out
-                    if (so == 0 && u >= 2 && !wait_all(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), abort_flag)) {
+                    if (so == 0 && u >= 2 && !wait_all<FITS>(dempty(acc), (uint32_t)(((u >> 1) - 1) & 1), abort_flag)) {
                         ok = false;
                         break;
                     }
                     for (int si = 0; si < nin; ++si) {
                         const int s = so * nin + si;
-                        if (h == 0 && !wait_all(afull(st), full, abort_flag)) { ok = false; break; }
+                        if (h == 0 && !wait_all<FITS>(afull(st), full, abort_flag)) { ok = false; break; }
                         tc_fence_after();
                         if (lead) {
                             issue_planes(L, sbase, st, s, boff, n, tmem + (uint32_t)(ND * n0 * acc));
@@ -510,7 +517,7 @@ __device__ __forceinline__ void split_pipeline(const SplitLayout &L, unsigned ch
         const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         for (int u = 0; u < nu; ++u) {
             const int c = u / nh, h = u % nh, acc = u & 1;
-            if (!wait_all(dfull(acc), (uint32_t)((u >> 1) & 1), abort_flag)) break;
+            if (!wait_all<FITS>(dfull(acc), (uint32_t)((u >> 1) & 1), abort_flag)) break;
             tc_fence_after();
             const int n = h ? n1 : n0, e0 = (warp >> 2) * (n / 2), e1 = min(e0 + n / 2, jm - kHalf * h);
             const uint32_t base = lanes + (uint32_t)(ND * n0 * acc);
@@ -594,7 +601,7 @@ __device__ __noinline__ void row_to_fp64(u64 *row, int ld, int e, int *rexp)
     if (threadIdx.x == 0) *rexp = kWideRow;
 }
 
-template <typename Ti>
+template <typename Ti, bool FITS>
 __global__ void __launch_bounds__(kThreads, 1)
 mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, u64 *ct, int *rexp, double *__restrict__ Z,
                         int z0, int W, int jbase, int rows, int drop)
@@ -639,7 +646,7 @@ mixed_gemm_split_kernel(const MixedArgs P, const Ti *__restrict__ astr, u64 *ct,
     src.z0 = z0;
     src.nsl = L.kp / kKS;
     src.nq = ncb * src.nsl;
-    split_pipeline(L, smem, sbase, tmem, ncb, jm, zchunk(Z, a, P.M, W, 0) + jbase * kM, P.M, src,
+    split_pipeline<FITS>(L, smem, sbase, tmem, ncb, jm, zchunk(Z, a, P.M, W, 0) + jbase * kM, P.M, src,
                    &abort_flag, a == drop);
     split_end(tmem, cols);
     if (abort_flag)   // uniform: written before split_end's barrier
@@ -670,8 +677,9 @@ int mixed_gemm_split(const MixedArgs &ma, const Ti *astr, double *ct, int *rexp,
     // BSIM_SPLIT_DROP_ROW (tests): the producers of this row fill nothing, so the row's
     // waits run out
     const char *drop = getenv("BSIM_SPLIT_DROP_ROW");
-    const size_t smem = split_layout(ma.nF, std::min(rows, ma.M - jbase), kMixTab).total;
-    auto kern = mixed_gemm_split_kernel<Ti>;
+    const SplitLayout L = split_layout(ma.nF, std::min(rows, ma.M - jbase), kMixTab);
+    const size_t smem = L.total;
+    auto kern = L.kp / kKS <= L.stages ? mixed_gemm_split_kernel<Ti, true> : mixed_gemm_split_kernel<Ti, false>;
     BSIM_CUDA(allow_smem(kern));
     launch_chained(kern, ma.nA, kThreads, smem, s, ma, astr, reinterpret_cast<u64 *>(ct), rexp, Z, z0, W, jbase, rows,
                    drop ? atoi(drop) : -1);

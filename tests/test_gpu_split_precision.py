@@ -120,3 +120,32 @@ def test_a_wait_that_runs_out_costs_no_result(cuda, system, monkeypatch):
     f.hvec(x, w)
     assert cuda.equal(w, z)
     assert timeouts(0) == 0
+
+
+@pytest.mark.parametrize("count", [1, 2, 30, 147, 149, 286])
+def test_wide_rows_among_others(cuda, monkeypatch, count):
+    """A few rows that stay in FP64 share their column chunks among the CTAs, many take one each: 286 rows of 715 columns
+    (six chunks), K of 78, thirty singles a row; the rows' elements spread over nine decades, their largest as the others'."""
+    from binsim_b200 import cuotf, network as nw
+    norb, na, nb = 13, 3, 4
+    B = cuotf.CuBasis(norb, na, nb)
+    f = cuotf.CuOTFFunctions(B, cuotf.CuNetwork(nw.hamiltonian_network(norb, seed=3, native=True)))
+    rng = np.random.default_rng(count)
+    x = rng.normal(size=(286, 715))
+    rows = rng.permutation(286)[:count]
+    x[rows] *= 10.0 ** rng.uniform(-9, 0, (count, 715))
+    x = dev(cuda, x.ravel())
+    y, z = cuda.full_like(x, float("nan")), cuda.empty_like(x)
+    monkeypatch.setenv("BSIM_SIGMA_SPLIT", "0")
+    f.hvec(x, z)
+    monkeypatch.setenv("BSIM_SIGMA_SPLIT", "1")
+    f.hvec(x, y)
+    assert float((y - z).abs().max()) <= 1e-13 * float(z.abs().max())
+    if count == 286:
+        assert cuda.equal(y, z)
+    # two windows of Z and column bands find the rows again
+    nB = 715
+    w = cuda.full_like(x, float("nan"))
+    for lo, hi in ((0, 384), (384, nB)):
+        f.hvec_cols(x, w, lo, hi)
+    assert float((y - w).abs().max()) <= 1e-13 * float(z.abs().max())

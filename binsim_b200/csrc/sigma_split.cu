@@ -47,9 +47,9 @@
 // accumulator is read out during the other's MMAs, and the epilogue's eight rows at a
 // time (8 loads per 8 rows, not per 4): 4.5 -> 3.8 ms; before that, biased words
 // (bytes d + 128: a subtraction negates them) and byte offsets in the gather table.
-// Against mixed_dmma_kernel, which runs at the FP64 tensor rate: 0.426 -> 0.35 ms at
-// 12o 6+6, 1.05 -> 0.80 ms at 13o 7+5, 5.72 -> 3.83 ms at 14o 7+7, 99.8 -> 67.7 ms at
-// 16o 8+8, 1.29 -> 0.83 ms at 20o 3+3.  On a vector whose rows all stay in FP64 (six
+// Against mixed_dmma_kernel, which runs at the FP64 tensor rate: 0.426 -> 0.343 ms at
+// 12o 6+6, 1.05 -> 0.78 ms at 13o 7+5, 5.72 -> 3.86 ms at 14o 7+7, 99.8 -> 68.5 ms at
+// 16o 8+8, 1.29 -> 0.82 ms at 20o 3+3 (with the launch for rows left in FP64).  On a vector whose rows all stay in FP64 (six
 // decades under a leading determinant, 13o 7+5) a sigma takes 2.16 ms, all rows split
 // 1.87.
 // Measured and not kept: FP16 digits (seven of 9 bits, kind::f16; 110 ms at 16o, for the

@@ -49,9 +49,9 @@
 // (bytes d + 128: a subtraction negates them) and byte offsets in the gather table.
 // Against mixed_dmma_kernel, which runs at the FP64 tensor rate: 0.426 -> 0.343 ms at
 // 12o 6+6, 1.05 -> 0.78 ms at 13o 7+5, 5.72 -> 3.86 ms at 14o 7+7, 99.8 -> 68.5 ms at
-// 16o 8+8, 1.29 -> 0.82 ms at 20o 3+3 (with the launch for rows left in FP64).  On a vector whose rows all stay in FP64 (six
-// decades under a leading determinant, 13o 7+5) a sigma takes 2.16 ms, all rows split
-// 1.87.
+// 16o 8+8, 1.29 -> 0.82 ms at 20o 3+3, with the launch for rows left in FP64.  On a vector
+// whose rows all stay in FP64 (six decades under a leading determinant, 13o 7+5) a sigma
+// takes 2.16 ms, with all rows split 1.87.
 // Measured and not kept: FP16 digits (seven of 9 bits, kind::f16; 110 ms at 16o, for the
 // conversion of the digits), the same kernel for the doubles through intermediate
 // strings (43 -> 50 ms at 16o: 45 rows of 64, K of 45 in 64, coalesced DMMA operands)
